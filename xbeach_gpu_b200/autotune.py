@@ -4,8 +4,8 @@ The batched kernels are persistent: each launch runs a chosen number of
 blocks that walk contiguous runs of the (scenario, tile) work list of its
 tile shape.  The best number depends on the kernel's occupancy, the number of
 work items and how ragged the scenarios are, and on which implementation
-runs: the wave rows pass has TMA plane tiles with one or two cells per thread
-(32 x 8 cells on 256 or 128 threads) and thread-copied tiles; the flow step's
+runs: the wave rows pass has TMA plane tiles (neighbouring cells per thread)
+and thread-copied tiles (one cell per thread); the flow step's
 momentum updates run fused into one pass or split in two (a fusion split);
 and the passes that read only a cell and its nearest neighbours (wavforce,
 the depth/viscosity and momentum passes, the first sediment pass) run in

@@ -15,8 +15,7 @@
 #include "../../include/xbg.h"
 #include "../../include/xbg_io.h"
 
-// the wave rows variant a new handle or batch starts with (1: TMA tiles, one
-// cell per thread; 2: TMA tiles, two cells per thread)
+// the wave rows variant a new handle or batch starts with (1, 2: TMA tiles)
 #ifndef XBG_WAVE_VARIANT_DEFAULT
 #define XBG_WAVE_VARIANT_DEFAULT 1
 #endif
@@ -27,7 +26,7 @@
 #endif
 
 namespace xbg {
-template <class R> int launch_wave(const Dev<R>&, const Konst<R>&, cudaStream_t, Prof*, cudaEvent_t, const WaveMaps*, int,
+template <class R> int launch_wave(const Dev<R>&, const Konst<R>&, cudaStream_t, Prof*, cudaEvent_t, const WaveMaps*,
                                    bool);
 template <class R> int wave_maps_make(const Dev<R>&, const Konst<R>&, WaveMaps*);
 template <class R> int wave_parts(const Konst<R>&);
@@ -44,7 +43,8 @@ template <class R> int launch_wavebnd_batch(const BatchTab<R>&, const BatchLaunc
 template <class R> int launch_ubnd_batch(const BatchTab<R>&, const BatchLaunch&, cudaStream_t, Prof*);
 template <class R> int launch_means_batch(const BatchTab<R>&, const BatchLaunch&, cudaStream_t, Prof*);
 template <class R> int launch_wave_batch(const BatchTab<R>&, const BatchLaunch&, int, int, int, cudaStream_t, Prof*,
-                                         cudaEvent_t, const WaveMaps*, int, bool);
+                                         cudaEvent_t, const WaveMaps*,
+                                   bool);
 template <class R> int launch_flow_batch(const BatchTab<R>&, const BatchLaunch&, cudaStream_t, Prof*, bool, bool);
 template <class R> int launch_sed_batch(const BatchTab<R>&, const BatchLaunch&, cudaStream_t, Prof*, bool);
 template <class R> int ubnd_threads(const Konst<R>&);
@@ -316,14 +316,13 @@ struct Handle : public xbg_handle {
     int nwave = 0;
     cudaError_t last_err = cudaSuccess;
     double* mass_buf = nullptr;
-    // wave rows pass: TMA tiles with one cell per thread (variant 1) or two
-    // (variant 2), when its maps could be made and wave-current interaction
-    // is off, or thread-copied tiles (variant 0)
+    // wave rows pass: TMA tiles (variants 1 and 2: one kernel), when its maps
+    // could be made and wave-current interaction is off, or thread-copied tiles
+    // (variant 0)
     WaveMaps maps;
     bool maps_ok = false;
     int wave_variant = XBG_WAVE_VARIANT_DEFAULT;
     const WaveMaps* wave_maps() const { return (maps_ok && wave_variant >= 1) ? &maps : nullptr; }
-    int wave_cpt() const { return wave_variant == 2 ? 2 : 1; }
     // flow: momentum steps in one pass (variant 1) or two (variant 0)
     int flow_variant = XBG_FLOW_VARIANT_DEFAULT;
     // the pointwise passes in 32 x 8 (variant 0) or 64 x 4 (variant 1) blocks,
@@ -700,11 +699,11 @@ struct Handle : public xbg_handle {
             n += launch_wavebnd(S, K, ser, side, nullptr, 0);
             if (K.flow == 1) n += launch_ubnd(S, K, ser, side, nullptr);
             cudaEventRecord(ev_join, side);
-            n += launch_wave(S, K, st, nullptr, ev_join, wave_maps(), wave_cpt(), wide());
+            n += launch_wave(S, K, st, nullptr, ev_join, wave_maps(), wide());
         } else {
             if (K.swave == 1) n += launch_wavebnd(S, K, ser, st, pf, 0);
             if (K.flow == 1) n += launch_ubnd(S, K, ser, st, pf);
-            if (K.swave == 1) n += launch_wave(S, K, st, pf, nullptr, wave_maps(), wave_cpt(), wide());
+            if (K.swave == 1) n += launch_wave(S, K, st, pf, nullptr, wave_maps(), wide());
         }
         if (K.flow == 1) n += launch_flow(S, K, st, pf, flow_variant == 1, wide(), vec());
         if (P.sedtrans == 1) n += launch_sed(S, K, st, pf, wide(), vec());
@@ -752,7 +751,7 @@ struct Handle : public xbg_handle {
             case 1: if (K.swave == 1) n = launch_wavebnd(S, K, ser, st, nullptr, 1); break;
             case 2: if (K.flow == 1) n = launch_ubnd(S, K, ser, st, nullptr); break;
             case 3:
-                if (K.swave == 1) n = launch_wave(S, K, st, nullptr, nullptr, wave_maps(), wave_cpt(), wide());
+                if (K.swave == 1) n = launch_wave(S, K, st, nullptr, nullptr, wave_maps(), wide());
                 break;
             case 4: if (K.flow == 1) n = launch_flow(S, K, st, nullptr, flow_variant == 1, wide(), vec()); break;
             case 5: if (P.sedtrans == 1) n = launch_sed(S, K, st, nullptr, wide(), vec()); break;
@@ -1041,7 +1040,6 @@ struct Batch : public xbg_batch {
     WaveMaps* dmaps = nullptr;            // the scenarios' tensor maps (TMA rows pass), if every scenario has them
     int wave_variant = XBG_WAVE_VARIANT_DEFAULT;   // 1, 2: TMA rows pass (when dmaps), 0: thread-copied tiles
     const WaveMaps* wave_maps() const { return wave_variant >= 1 ? dmaps : nullptr; }
-    int wave_cpt() const { return wave_variant == 2 ? 2 : 1; }
     int tile_variant = 0;   // the pointwise passes over 32 x 8 (0) or 64 x 4 (1) tiles
     bool wide() const { return tile_variant == 1; }
     int flow_variant = XBG_FLOW_VARIANT_DEFAULT;   // 1: momentum steps in one pass, 0: two
@@ -1171,12 +1169,12 @@ struct Batch : public xbg_batch {
             k += launch_wavebnd_batch(T, L, side, nullptr);
             if (flow == 1) k += launch_ubnd_batch(T, L, side, nullptr);
             cudaEventRecord(ev_join, side);
-            k += launch_wave_batch(T, L, nt, roller, wci, st, nullptr, ev_join, wave_maps(), wave_cpt(), wide());
+            k += launch_wave_batch(T, L, nt, roller, wci, st, nullptr, ev_join, wave_maps(), wide());
         } else {
             if (swave == 1) k += launch_wavebnd_batch(T, L, st, pf);
             if (flow == 1) k += launch_ubnd_batch(T, L, st, pf);
             if (swave == 1)
-                k += launch_wave_batch(T, L, nt, roller, wci, st, pf, nullptr, wave_maps(), wave_cpt(), wide());
+                k += launch_wave_batch(T, L, nt, roller, wci, st, pf, nullptr, wave_maps(), wide());
         }
         return k;
     }

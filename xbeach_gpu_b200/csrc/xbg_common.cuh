@@ -93,7 +93,8 @@ enum Fld {
 // Per-step temporaries (never read across steps).
 enum Tmp {
     T_UU = 0, T_VV, T_ZS, T_NUH, T_SXX, T_SXY, T_SYY, T_CEQBG, T_TSG, T_UA, T_FACERO,
-    T_ERO, T_DEPO, T_ZB, T_STDEP, T_HH, T_QX, T_QY, NTMP
+    T_ERO, T_DEPO, T_ZB, T_STDEP, T_HH, T_QX, T_QY, NTMP,
+    T_SIG = T_CEQBG   // sigma / sinh(2 kh), dispersion pass to rows pass (the sediment step overwrites it)
 };
 
 template <class R>
@@ -172,10 +173,10 @@ struct Konst {
 };
 
 // Tensor maps of the wave rows pass (TMA variant): ee and rr of both plane
-// sets, box loads of one bin's plane tile and box stores of all bins of a
-// block's cells.  Passed to the kernel as a __grid_constant__ parameter.
+// sets, box loads of one bin's plane tile.  Passed to the kernel as a
+// __grid_constant__ parameter.
 struct WaveMaps {
-    CUtensorMap ld_e[2], ld_r[2], st_e[2], st_r[2];
+    CUtensorMap ld_e[2], ld_r[2];
 };
 
 // Per-kernel timing of a non-graph step (xbg_profile_step): an event after
