@@ -24,6 +24,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/xbg.h"
 #include "../../include/xbg_nn.h"
@@ -423,7 +424,9 @@ __global__ void __launch_bounds__(256, 2) k_conv_tc(const __nv_bfloat16* __restr
 // zero-filled by the threads.  No multicast; the map covers this GPU's
 // memory only.
 template <int WC>
-__host__ __device__ constexpr uint32_t sw_layout() { return WC == 32 ? 4u : 6u; }   // SWIZZLE_64B / SWIZZLE_32B
+__host__ __device__ constexpr uint32_t sw_layout() {   // SWIZZLE_128B / 64B / 32B
+    return WC == 64 ? 2u : (WC == 32 ? 4u : 6u);
+}
 
 template <int WC>
 __device__ __forceinline__ uint64_t swk_desc(unsigned saddr) {   // K-major, rows of WC*2 bytes
@@ -618,28 +621,35 @@ __global__ void __launch_bounds__(256, 2) k_conv_tma(const __grid_constant__ CUt
 // box (WC, Wt, R, 1) with the WC*2-byte swizzle; false when the shape does
 // not tile (W neither a multiple nor a divisor of 128, H not a multiple of R,
 // channel counts not multiples of WC, strides not 16-byte multiples).
-template <int WC>
-bool conv_map(const void* X, int B, int H, int W, int cin, int ldx, CUtensorMap* m) {
+inline PFN_cuTensorMapEncodeTiled_v12000 map_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
-    if (cin % WC || ldx % 8) return false;
-    const int Wt = W >= GM ? GM : W;
-    if (W >= GM ? (W % GM) : (GM % W)) return false;
-    const int R = GM / Wt;
-    if (H % R) return false;
     if (!enc) {
         cudaDriverEntryPointQueryResult q;
         void* fn = nullptr;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
             q != cudaDriverEntryPointSuccess || !fn)
-            return false;
+            return nullptr;
         enc = (PFN_cuTensorMapEncodeTiled_v12000)fn;
     }
+    return enc;
+}
+template <int WC>
+bool conv_map(const void* X, int B, int H, int W, int cin, int ldx, CUtensorMap* m) {
+    if (cin % WC || ldx % 8) return false;
+    const int Wt = W >= GM ? GM : W;
+    if (W >= GM ? (W % GM) : (GM % W)) return false;
+    const int R = GM / Wt;
+    if (H % R) return false;
+    PFN_cuTensorMapEncodeTiled_v12000 enc = map_encoder();
+    if (!enc) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)ldx, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
     const cuuint64_t strides[3] = {(cuuint64_t)ldx * 2, (cuuint64_t)W * ldx * 2, (cuuint64_t)H * W * ldx * 2};
     const cuuint32_t box[4] = {(cuuint32_t)WC, (cuuint32_t)Wt, (cuuint32_t)R, 1};
     const cuuint32_t es[4] = {1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(X), dims, strides, box, es,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, WC == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, WC == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+               : WC == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                          : CU_TENSOR_MAP_SWIZZLE_32B,
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -661,6 +671,482 @@ int conv_tma_launch(const CUtensorMap& m, const void* Wt, const float* bias, voi
     return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA;
 }
 
+// A bounded wait of one role of a warp-specialised kernel, which also ends when
+// another role has given up (bad, in shared memory).
+__device__ __forceinline__ bool role_wait(unsigned a, unsigned parity, int* bad) {
+    if (mbar_wait(a, parity, 64)) return true;
+#pragma unroll 1
+    for (int k = 0; k < 1024; k++) {
+        if (mbar_wait(a, parity, WAIT_LIMIT / 1024)) return true;
+        if (*(volatile int*)bad) return false;
+    }
+    *(volatile int*)bad = 1;
+    return false;
+}
+// CW accumulator columns of this warp's 32 tensor-memory lanes (one pixel per
+// lane) in registers
+template <int CW>
+__device__ __forceinline__ void load_cols(unsigned (&v)[CW], unsigned taddr) {
+#pragma unroll
+    for (int h = 0; h < CW; h += 8)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                     : "=r"(v[h]), "=r"(v[h + 1]), "=r"(v[h + 2]), "=r"(v[h + 3]), "=r"(v[h + 4]), "=r"(v[h + 5]),
+                       "=r"(v[h + 6]), "=r"(v[h + 7])
+                     : "r"(taddr + (unsigned)h));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+// ... plus bias, ReLU, to element `at` of Y (bf16 or fp32)
+template <int CW>
+__device__ __forceinline__ void put_cols(const unsigned (&v)[CW], const float* bias, void* Y, size_t at, int flags) {
+    float f[CW];
+#pragma unroll
+    for (int j = 0; j < CW; j++) {
+        f[j] = __uint_as_float(v[j]) + (bias ? bias[j] : 0.0f);
+        if (flags & XBG_NN_RELU) f[j] = fmaxf(f[j], 0.0f);
+    }
+    if (flags & XBG_NN_OUT_BF16) {
+        __align__(16) __nv_bfloat16 h[CW];
+#pragma unroll
+        for (int j = 0; j < CW; j++) h[j] = __float2bfloat16(f[j]);
+        uint4* d = (uint4*)((__nv_bfloat16*)Y + at);
+#pragma unroll
+        for (int j = 0; j < CW / 8; j++) d[j] = ((const uint4*)h)[j];
+    } else {
+        float4* d = (float4*)((float*)Y + at);
+#pragma unroll
+        for (int j = 0; j < CW / 4; j++) d[j] = ((const float4*)f)[j];
+    }
+}
+template <int CW>
+__device__ __forceinline__ void store_cols(unsigned taddr, const float* bias, void* Y, size_t at, int flags) {
+    unsigned v[CW];
+    load_cols<CW>(v, taddr);
+    put_cols<CW>(v, bias, Y, at, flags);
+}
+
+// ------------------------------------------------------------------------
+// The forward convolution over rows of 128 pixels, for layers whose weights
+// fit in shared memory beside the input stages (W a multiple of 128, N <= 128).
+// k_conv_tma loads an output tile's input nine times, once per tap, and starts
+// and drains a pipeline for every 128 pixels: its time is the copies' latency.
+// Here
+//  - a CTA (one per SM) takes a contiguous run of output rows of 128 pixels and
+//    keeps the layer's weights in shared memory for all of them;
+//  - it streams the input rows of its strip downwards, each as three boxes (one
+//    per dx; 128 pixels x WC channels x cin / WC), and uses a box for the three
+//    output rows that see it before it leaves: input row r is tap row 0 of
+//    output row r+1, 1 of r and 2 of r-1.  So the input crosses L2 three times
+//    instead of nine, and every accumulator still adds its products in the order
+//    tap, channel: the results are those of the other kernels bit for bit;
+//  - the accumulators of consecutive output rows rotate through NS slots of
+//    tensor memory, so that the epilogue of one row runs beside the next rows'
+//    products.
+// Warp 0 issues the copies, warp 1 the products, warps 2..5 store the rows; all
+// meet on mbarriers (full / empty per stage and per accumulator slot).  Every
+// wait is bounded: a role that gives up sets a flag that ends the others' waits,
+// and the CTA leaves after its copies and products in flight (bounded again).
+// At 512 x 1024 pixels, against k_conv_tma: 32 -> 32 channels 65 -> 32 us, 96 -> 32
+// 147 -> 66, 16 -> 32 52 -> 27; at 256 x 512, 64 -> 64 38 -> 20.  What is left is
+// the issue of the products: 55 to 90 cycles each at 16 to 64 output channels.
+constexpr int CR_MAXST = 18;      // input stages at most
+constexpr int CR_THREADS = 192;
+
+template <int BN>
+struct ConvRows {
+    // accumulator slots (three rows under way, at least one being stored) of
+    // STRIDE tensor-memory columns
+    static constexpr int STRIDE = BN <= 32 ? 32 : (BN <= 64 ? 64 : 128);
+    static constexpr int NS = BN <= 64 ? 8 : 4;
+    static constexpr int COLS = NS * STRIDE;
+};
+
+template <int BN, int WC>
+__global__ void __launch_bounds__(CR_THREADS, 1)
+    k_conv_rows(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* __restrict__ Wt,
+                const float* __restrict__ bias, void* Y, int Bn, int H, int W, int cin, int ldw, int ldy, int flags,
+                int nst, int* err) {
+    constexpr int NS = ConvRows<BN>::NS, STRIDE = ConvRows<BN>::STRIDE, TCOLS = ConvRows<BN>::COLS;
+    constexpr int BOX = GM * WC * 2;              // bytes of a box: 128 pixels of WC channels
+    constexpr int CHUNK = BN * WC * 2;            // bytes of the weights of one tap and channel group
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long full[CR_MAXST], empty[CR_MAXST], afull[NS], aempty[NS], drain;
+    __shared__ unsigned tmem_slot;
+    __shared__ int bad;
+    __shared__ float sbias[BN];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int strips = W / GM, total = Bn * strips * H, ncg = cin / WC, nb = 3 * ncg;   // boxes of an input row
+    const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int lo = (int)blockIdx.x * per, hi = min(total, lo + per);
+    if (lo >= hi) return;   // the whole CTA
+    const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const unsigned wbase = base + (unsigned)nst * BOX;   // the weights, [tap][channel group][BN][WC]
+
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(TCOLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    if (tid == 0) {
+        bad = 0;
+        for (int s = 0; s < nst; s++) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
+        for (int s = 0; s < NS; s++) { mbar_init(smem_u32(&afull[s]), 1); mbar_init(smem_u32(&aempty[s]), 4); }
+        mbar_init(smem_u32(&drain), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (tid < BN) sbias[tid] = bias ? bias[tid] : 0.0f;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp > 0) {   // the weights, K-major rows of WC channels with the swizzle of the boxes; the copies start meanwhile
+        for (int q = tid - 32; q < 9 * ncg * BN * (WC / 8); q += CR_THREADS - 32) {
+            const int c = q % (WC / 8), rk = q / (WC / 8), r = rk % BN, kc = rk / BN;
+            const unsigned lin = (unsigned)(r * WC * 2 + c * 16);
+            cp16(wbase + (unsigned)kc * CHUNK + (lin ^ (((lin >> 7) & (WC == 64 ? 7u : (WC == 32 ? 3u : 1u))) << 4)),
+                 Wt + (size_t)r * ldw + kc * WC + c * 8);
+        }
+        asm volatile("cp.async.commit_group;\ncp.async.wait_all;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        asm volatile("bar.sync 1, %0;\n" ::"n"(CR_THREADS - 32) : "memory");
+    }
+    const unsigned tmem = tmem_slot;
+    unsigned leader;   // one lane of each warp
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
+    auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
+    // The run's segments (rows of one strip of one image) in order:
+    // seg(b, x0, y0, n, o0) with o0 the number of the segment's first row in
+    // the run; returns false to stop.
+    auto segments = [&](auto&& seg) {
+        for (int l = lo; l < hi;) {
+            const int y0 = l % H, sb = l / H, n = min(hi - l, H - y0);
+            if (!seg(sb / strips, (sb % strips) * GM, y0, n, l - lo)) return;
+            l += n;
+        }
+    };
+    if (warp == 0) {
+        // ---- copies: lane c takes box c of an input row (dx, channel group)
+        const int cx = lane / ncg - 1, cch = lane % ncg * WC;
+        int s = 0, mine = -1;   // the row's first stage; the stage this lane used last
+        unsigned ph = 0, minep = 0;
+        segments([&](int b, int x0, int y0, int n, int) {
+            for (int r = y0 - 1; r <= y0 + n; r++) {
+                bool ok = true;
+                if (lane < nb) {
+                    const int t = s + lane < nst ? s + lane : s + lane - nst;
+                    const unsigned tp = s + lane < nst ? ph : ph ^ 1u;
+                    ok = wait(smem_u32(&empty[t]), tp ^ 1u);
+                    if (ok) {
+                        const unsigned fb = smem_u32(&full[t]);
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb),
+                                     "r"((unsigned)BOX)
+                                     : "memory");
+                        asm volatile(
+                            "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                            "[%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(base + (unsigned)t * BOX),
+                            "l"((unsigned long long)&xmap), "r"(cch), "r"(x0 + cx), "r"(r), "r"(b), "r"(fb)
+                            : "memory");
+                        mine = t;
+                        minep = tp;
+                    }
+                }
+                if (!__all_sync(0xffffffffu, ok)) return false;
+                s += nb;
+                if (s >= nst) { s -= nst; ph ^= 1u; }
+            }
+            return true;
+        });
+        // leaving early: every stage's copy in flight lands first.  A lane's last
+        // box lands after its earlier ones have been waited for by the products
+        // or are older than it in the same queue; the bounded wait covers both.
+        if (*(volatile int*)&bad && mine >= 0) mbar_wait(smem_u32(&full[mine]), minep);
+    } else if (warp == 1) {   // ---- products: the warp runs in step, one lane issues
+        const uint32_t idesc = idesc_bf16(GM, BN);
+        const uint64_t da0 = swk_desc<WC>(base), db0 = swk_desc<WC>(wbase);
+        const uint64_t tstep = (uint64_t)(3 * ncg * CHUNK >> 4);   // from a tap row's weights to the next one's
+        auto commit = [&](const void* bar) {
+            if (leader) asm volatile(
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar))
+                : "memory");
+        };
+        auto mma = [&](unsigned d, uint64_t da, uint64_t db, unsigned acc) {
+            if (leader) asm volatile(
+                "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+                "l"(da), "l"(db), "r"(idesc), "r"(acc));
+        };
+        int s = 0;
+        unsigned ph = 0;
+        segments([&](int, int, int y0, int n, int o0) {
+            for (int r = y0 - 1; r <= y0 + n; r++) {
+                const int on = o0 + r + 1 - y0;   // the output row that starts here, if any
+                const bool v0 = r + 1 < y0 + n, v1 = r >= y0 && r < y0 + n, v2 = r - 1 >= y0;
+                // the row's boxes and, for the row that starts, its accumulator: one
+                // lane waits for each
+                bool ok = true;
+                if (lane < nb)
+                    ok = wait(smem_u32(&full[s + lane < nst ? s + lane : s + lane - nst]), s + lane < nst ? ph : ph ^ 1u);
+                else if (lane == 31 && v0)
+                    ok = wait(smem_u32(&aempty[on % NS]), ((unsigned)(on / NS) & 1u) ^ 1u);
+                if (!__all_sync(0xffffffffu, ok)) return false;
+                tc_fence_after();
+                // accumulators of the output rows that see this input row as tap row 0, 1, 2
+                const unsigned d0 = tmem + (unsigned)((on + NS) % NS) * STRIDE, d1 = tmem + (unsigned)((on - 1 + NS) % NS) * STRIDE,
+                               d2 = tmem + (unsigned)((on - 2 + NS) % NS) * STRIDE;
+                // dx, channel group; inner: all three output rows exist
+                auto boxes = [&](auto inner) {
+                    constexpr bool IN = decltype(inner)::value;
+                    uint64_t db = db0;
+                    int t = s;
+                    for (int c = 0; c < nb; c++) {
+                        const uint64_t da = da0 + (uint64_t)((unsigned)t * BOX >> 4);
+#pragma unroll
+                        for (int j = 0; j < WC / 16; j++) {
+                            // the row that starts here: its first product overwrites
+                            if (IN || v0) mma(d0, da + 2 * j, db + 2 * j, j || c ? 1u : 0u);
+                            if (IN || v1) mma(d1, da + 2 * j, db + tstep + 2 * j, 1u);
+                            if (IN || v2) mma(d2, da + 2 * j, db + 2 * tstep + 2 * j, 1u);
+                        }
+                        commit(&empty[t]);
+                        db += CHUNK >> 4;
+                        if (++t == nst) t = 0;
+                    }
+                };
+                if (v0 && v1 && v2) boxes(std::true_type{});
+                else boxes(std::false_type{});
+                s += nb;
+                if (s >= nst) { s -= nst; ph ^= 1u; }
+                if (v2) commit(&afull[(on - 2 + NS) % NS]);   // output row r-1 has all its taps
+            }
+            return true;
+        });
+        if (*(volatile int*)&bad) {   // products in flight end before tensor memory goes
+            commit(&drain);
+            mbar_wait(smem_u32(&drain), 0);
+        }
+    } else {   // ---- rows out: warp w reads tensor memory lanes 32 (w % 4) ..
+        const int q = warp & 3;
+        segments([&](int b, int x0, int y0, int n, int o0) {
+            for (int y = y0; y < y0 + n; y++) {
+                const int o = o0 + y - y0, slot = o % NS;
+                if (!__all_sync(0xffffffffu, wait(smem_u32(&afull[slot]), (unsigned)(o / NS) & 1u))) return false;
+                tc_fence_after();
+                const size_t row = (size_t)(b * H + y) * W + x0 + q * 32 + lane;
+                constexpr int CW = BN % 32 == 0 ? 32 : 16;   // columns at a time
+#pragma unroll
+                for (int c0 = 0; c0 < BN; c0 += CW) {
+                    unsigned v[CW];
+                    load_cols<CW>(v, tmem + ((unsigned)(q * 32) << 16) + (unsigned)(slot * STRIDE + c0));
+                    if (c0 + CW >= BN) {   // the slot is read: the next row may start in it
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0)
+                            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(&aempty[slot]))
+                                         : "memory");
+                    }
+                    put_cols<CW>(v, sbias + c0, Y, row * ldy + c0, flags);
+                }
+            }
+            return true;
+        });
+    }
+    __syncthreads();
+    if (tid == 0 && bad) atomicExch(err, XBG_ERR_TIMEOUT);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS));
+}
+
+// stages that fit beside the weights of a layer (0: k_conv_rows does not apply)
+template <int BN, int WC>
+int conv_rows_stages(int W, int cin) {
+    if (BN > 128 || W % GM) return 0;
+    const int room = 225 * 1024 - 1024 - 9 * cin * BN * 2, box = GM * WC * 2;
+    const int n = room < 0 ? 0 : room / box;
+    const int nb = 3 * (cin / WC);   // an input row's boxes are waited for together; two rows' worth, or nearly
+    return nb > 30 || n < nb + (nb + 1) / 2 ? 0 : (n > CR_MAXST ? CR_MAXST : n);
+}
+
+template <int BN, int WC>
+int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
+                     int ldw, int ldy, int flags, int nst, int* err, cudaStream_t st) {
+    static int sms = 0;   // attribute and SM count: the same for every caller
+    if (!sms) {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaFuncSetAttribute(k_conv_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024) !=
+                cudaSuccess)
+            return XBG_ERR_CUDA;
+        sms = n;
+    }
+    const long long total = (long long)Bn * (W / GM) * H;
+    const size_t smem = 1024 + (size_t)nst * GM * WC * 2 + (size_t)9 * cin * BN * 2;
+    k_conv_rows<BN, WC><<<(unsigned)(total < sms ? total : sms), CR_THREADS, smem, st>>>(
+        m, (const __nv_bfloat16*)Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err);
+    return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA;
+}
+
+// ------------------------------------------------------------------------
+// The forward convolution as k_conv_tma (the same products in the same order,
+// an output tile of 128 pixels x BN of the layer's channels per CTA) with a warp
+// for the copies, one for the products and four for the tile's store, for
+// inputs of a multiple of 64 channels.  k_conv_tma's threads meet twice per
+// 64-wide chunk and its next copies wait for the last chunk's products, so a
+// chunk takes about a microsecond whatever the stages; here the copies run
+// ahead as far as there are stages and the products never wait for a thread.
+// A chunk is one box of the input (64 channels of one tap, 128-byte swizzle)
+// and one of the weights ([BN][64]).  Waits as in k_conv_rows.  Against
+// k_conv_tma: 256 -> 256 channels at 64 x 128 pixels 50 -> 14 us, 384 -> 128 at
+// 128 x 256 69 -> 27, 192 -> 64 at 256 x 512 94 -> 47.
+template <int BN, int ST>
+__global__ void __launch_bounds__(192, 1)
+    k_conv_ws(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
+              const float* __restrict__ bias, void* Y, int Bn, int H, int W, int cin, int ldy, int flags, int* err) {
+    constexpr int A_BYTES = GM * GK * 2, B_BYTES = BN * GK * 2, STAGE = A_BYTES + B_BYTES;
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long full[ST], empty[ST], done;
+    __shared__ unsigned tmem_slot;
+    __shared__ int bad;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * GM, n0 = blockIdx.y * BN, nk = 9 * cin / GK;
+    const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(BN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    if (tid == 0) {
+        bad = 0;
+        for (int s = 0; s < ST; s++) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
+        mbar_init(smem_u32(&done), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = tmem_slot;
+    unsigned leader;   // one lane of each warp
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
+    auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
+    if (warp == 0) {   // ---- copies
+        const int HW = H * W, b = m0 / HW, rem = m0 - b * HW, y0 = rem / W, x0 = rem - y0 * W;
+        int s = 0, c0 = 0, dx = -1, dy = -1, kc = 0;
+        unsigned ph = 0;
+        for (; kc < nk; kc++) {
+            if (!wait(smem_u32(&empty[s]), ph ^ 1u)) break;
+            if (leader) {
+                const unsigned fb = smem_u32(&full[s]), sa = base + (unsigned)s * STAGE;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"((unsigned)STAGE)
+                             : "memory");
+                asm volatile(
+                    "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+                    "%3, %4, %5}], [%6];\n" ::"r"(sa),
+                    "l"((unsigned long long)&xmap), "r"(c0), "r"(x0 + dx), "r"(y0 + dy), "r"(b), "r"(fb)
+                    : "memory");
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+                    "%3}], [%4];\n" ::"r"(sa + A_BYTES),
+                    "l"((unsigned long long)&wmap), "r"(kc * GK), "r"(n0), "r"(fb)
+                    : "memory");
+            }
+            if (++s == ST) { s = 0; ph ^= 1u; }
+            c0 += GK;
+            if (c0 == cin) {
+                c0 = 0;
+                if (++dx == 2) { dx = -1; dy++; }
+            }
+        }
+        if (*(volatile int*)&bad)   // leaving early: the copies in flight land first (bounded)
+            for (int c = max(kc - ST, 0); c < kc; c++) mbar_wait(smem_u32(&full[c % ST]), (c / ST) & 1);
+    } else if (warp == 1) {   // ---- products
+        const uint32_t idesc = idesc_bf16(GM, BN);
+        const uint64_t a0 = sw128_desc(base), b0 = sw128_desc(base + A_BYTES);
+        int s = 0, kc = 0;
+        unsigned ph = 0;
+        for (; kc < nk; kc++) {
+            if (!wait(smem_u32(&full[s]), ph)) break;
+            tc_fence_after();
+            const uint64_t off = (uint64_t)((unsigned)s * STAGE >> 4);
+#pragma unroll
+            for (int j = 0; j < GK / 16; j++)
+                if (leader)
+                    asm volatile(
+                        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+                        "l"(a0 + off + 2 * j), "l"(b0 + off + 2 * j), "r"(idesc), "r"(j || kc ? 1u : 0u));
+            if (leader)
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                                 smem_u32(&empty[s]))
+                             : "memory");
+            if (++s == ST) { s = 0; ph ^= 1u; }
+        }
+        // every product issued so far (all of them, or those before a wait ran out)
+        if (leader)
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                             smem_u32(&done))
+                         : "memory");
+        if (*(volatile int*)&bad) mbar_wait(smem_u32(&done), 0);
+    } else {   // ---- the tile out
+        const int q = warp & 3;
+        if (__all_sync(0xffffffffu, wait(smem_u32(&done), 0)) && !*(volatile int*)&bad) {
+            tc_fence_after();
+            const size_t row = (size_t)m0 + q * 32 + lane;
+#pragma unroll 1
+            for (int c0 = 0; c0 < BN; c0 += 32)
+                store_cols<32>(tmem + ((unsigned)(q * 32) << 16) + (unsigned)c0, bias ? bias + n0 + c0 : nullptr, Y,
+                               row * ldy + n0 + c0, flags);
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && bad) atomicExch(err, XBG_ERR_TIMEOUT);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN));
+}
+
+// The tensor map of the weights, [rows][Kp] in boxes of BN rows x 64.
+inline bool weight_map(const void* Wt, int rows, int Kp, int ldw, int bn, CUtensorMap* m) {
+    PFN_cuTensorMapEncodeTiled_v12000 enc = map_encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ldw * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)GK, (cuuint32_t)bn}, es[2] = {1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(Wt), dims, strides, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN, int ST>
+int conv_ws_launch(const CUtensorMap& xm, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
+                   int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
+    constexpr size_t smem = (size_t)ST * (GM + BN) * GK * 2 + 1024;
+    static bool attr = false;
+    if (!attr) {
+        if (cudaFuncSetAttribute(k_conv_ws<BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess)
+            return XBG_ERR_CUDA;
+        attr = true;
+    }
+    CUtensorMap wm;
+    if (!weight_map(Wt, N, Kp, ldw, BN, &wm)) return XBG_ERR_CUDA;
+    const dim3 grid((unsigned)((long long)Bn * H * W / GM), (unsigned)(N / BN));
+    k_conv_ws<BN, ST><<<grid, 192, smem, st>>>(xm, wm, bias, Y, Bn, H, W, cin, ldy, flags, err);
+    return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA;
+}
+
+// BN of a CTA and its stages.  128 channels where the tiles then still fill most
+// SMs (the input is read once per slice), else slices of 64; one CTA per SM with
+// deep stages where the grid has no second wave, two with half of them elsewhere.
+inline int conv_ws(const CUtensorMap& xm, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
+                   int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
+    const long long tiles = (long long)Bn * H * W / GM;
+    const bool wide = N % 128 == 0 && tiles * (N / 128) >= 100;
+    const bool deep = tiles * (N / (wide ? 128 : 64)) <= 148;
+#define XBG_CONV_WS(BN, ST) \
+    conv_ws_launch<BN, ST>(xm, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st)
+    if (wide) return deep ? XBG_CONV_WS(128, 6) : XBG_CONV_WS(128, 3);
+    return deep ? XBG_CONV_WS(64, 8) : XBG_CONV_WS(64, 4);
+#undef XBG_CONV_WS
+}
+
 // whether xbg_nn_conv3x3 moves its input with box copies (test switch of the
 // thread-gathered path, xbg_nn_conv_set_tma)
 static int g_conv_tma = 1;
@@ -678,11 +1164,36 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
     }
     const long long M = (long long)Bn * H * W;
     if (g_conv_tma && M % GM == 0) {   // box copies of the input when the shape tiles
+        // over rows where the weights fit beside the stages (the input is read
+        // three times instead of nine), else tile by tile in 64-channel chunks,
+        // else (channel counts that are no multiple of 64) k_conv_tma
         CUtensorMap m;
-        if (cin % 32 == 0 && conv_map<32>(X, Bn, H, W, cin, ldx, &m))
+        if constexpr (BN <= 128) {
+            if (cin % 64 == 0) {
+                const int nst = conv_rows_stages<BN, 64>(W, cin);
+                if (nst && conv_map<64>(X, Bn, H, W, cin, ldx, &m))
+                    return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
+            }
+        }
+        if constexpr (BN % 64 == 0) {
+            if (cin % 64 == 0 && !(BN <= 128 && conv_rows_stages<(BN <= 128 ? BN : 128), 32>(W, cin)) &&
+                conv_map<64>(X, Bn, H, W, cin, ldx, &m))
+                return conv_ws(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
+        }
+        if (cin % 32 == 0 && conv_map<32>(X, Bn, H, W, cin, ldx, &m)) {
+            if constexpr (BN <= 128) {
+                const int nst = conv_rows_stages<BN, 32>(W, cin);
+                if (nst) return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
+            }
             return conv_tma_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
-        if (cin % 32 != 0 && conv_map<16>(X, Bn, H, W, cin, ldx, &m))
+        }
+        if (cin % 32 != 0 && conv_map<16>(X, Bn, H, W, cin, ldx, &m)) {
+            if constexpr (BN <= 128) {
+                const int nst = conv_rows_stages<BN, 16>(W, cin);
+                if (nst) return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
+            }
             return conv_tma_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
+        }
     }
     k_conv_tc<BN><<<(unsigned)((M + GM - 1) / GM), 256, smem, st>>>((const __nv_bfloat16*)X,
                                                                      (const __nv_bfloat16*)Wt, bias, Y, Bn, H, W, cin,
