@@ -20,6 +20,8 @@
 // has no effect on the state and is not evaluated.  Quotients by the grid
 // spacing are products with its reciprocal (within an ulp of the reference's
 // float division).
+#include <type_traits>
+
 #include "xbg_common.cuh"
 
 namespace xbg {
@@ -423,22 +425,28 @@ __device__ __forceinline__ R depth_face(R zsi, R zsn, R zbi, R zbn, R u, R eps) 
 // Fields of the momentum-correction pass, in its shared-memory tile.
 enum { C_ZS, C_ZB, C_UU, C_VV, C_UO, C_VO, C_QX, C_QY, C_NF };
 
+// min(level) + min(bed) > d over the window x in [x0, x1], y in [y0, y1]
+template <class R, class A>
+__device__ __forceinline__ bool zz_deeper(const A& a, int x0, int x1, int y0, int y1, R d) {
+    const Pair2<R> m = zz_min<R>(a, x0, x1, y0, y1);
+    return m.a + m.b > d;
+}
+
 // wrkuu2Ocorr (Flow_kernel.cu:1960-2044) at cell (ix, iy); a: field access
 // around the cell (uu is the post-Euler uu*, uo the previous step's).
-template <class R, class A>
+// DEEP: every window of the block is known to be deep enough.
+template <class R, bool DEEP, class A>
 __device__ __forceinline__ void wrk_u(const A& a, const Konst<R>& K, int ix, int iy, R& w1, R& w2) {
     const R eps2 = K.eps * (R)2.0f;
     w1 = (R)0.0f; w2 = (R)0.0f;
     if (ix > 0) {
-        const Pair2<R> m1 = zz_min<R>(a, -2, 2, 0, 0);   // zs, zb over x-2 .. x+2
-        if (m1.a + m1.b > eps2) {
+        if (DEEP || zz_deeper<R>(a, -2, 2, 0, 0, eps2)) {   // zs, zb over x-2 .. x+2
             R qs = a(C_QX, 0, 0) + a(C_QX, -1, 0);
             if (qs > (R)0.0f) w1 = (R)0.5f * minmod(a(C_UU, 0, 0) - a(C_UO, -1, 0), a(C_UU, -1, 0) - a(C_UO, -2, 0));
             if (qs < (R)0.0f) w1 = (R)-0.5f * minmod(a(C_UO, 0, 0) - a(C_UU, -1, 0), a(C_UO, 1, 0) - a(C_UU, 0, 0));
         }
         if (iy > 0) {
-            const Pair2<R> m2 = zz_min<R>(a, 0, 1, -1, 2);   // x, x+1 over y-1 .. y+2
-            if (m2.a + m2.b > eps2) {
+            if (DEEP || zz_deeper<R>(a, 0, 1, -1, 2, eps2)) {   // x, x+1 over y-1 .. y+2
                 R qs = a(C_QY, 1, 0) + a(C_QY, 0, 0);
                 if (qs > (R)0.0f) w2 = (R)0.5f * minmod(a(C_UU, 0, 1) - a(C_UO, 0, 0), a(C_UU, 0, 0) - a(C_UO, 0, -1));
                 if (qs < (R)0.0f) w2 = (R)-0.5f * minmod(a(C_UO, 0, 1) - a(C_UU, 0, 0), a(C_UO, 0, 2) - a(C_UU, 0, 1));
@@ -448,19 +456,17 @@ __device__ __forceinline__ void wrk_u(const A& a, const Konst<R>& K, int ix, int
 }
 
 // wrkvv2Ocorr (Flow_kernel.cu:2046-2128) at cell (ix, iy)
-template <class R, class A>
+template <class R, bool DEEP, class A>
 __device__ __forceinline__ void wrk_v(const A& a, const Konst<R>& K, int ix, int iy, R& w1, R& w2) {
     const R eps2 = K.eps * (R)2.0f;
     w1 = (R)0.0f; w2 = (R)0.0f;
     if (ix > 0 && iy > 0 && iy < K.ny - 2) {
-        const Pair2<R> m1 = zz_min<R>(a, 0, 0, -2, 2);   // y-2 .. y+2
-        if (m1.a + m1.b > eps2) {
+        if (DEEP || zz_deeper<R>(a, 0, 0, -2, 2, eps2)) {   // y-2 .. y+2
             R qs = a(C_QY, 0, 0) + a(C_QY, 0, -1);
             if (qs > (R)0.0f) w1 = (R)0.5f * minmod(a(C_VV, 0, 0) - a(C_VO, 0, -1), a(C_VV, 0, -1) - a(C_VO, 0, -2));
             if (qs < (R)0.0f) w1 = (R)-0.5f * minmod(a(C_VO, 0, 0) - a(C_VV, 0, -1), a(C_VO, 0, 1) - a(C_VV, 0, 0));
         }
-        const Pair2<R> m2 = zz_min<R>(a, -1, 2, 0, 1);   // x-1 .. x+2 over y, y+1
-        if (m2.a + m2.b > eps2) {
+        if (DEEP || zz_deeper<R>(a, -1, 2, 0, 1, eps2)) {   // x-1 .. x+2 over y, y+1
             R qs = a(C_QX, 0, 1) + a(C_QX, 0, 0);
             if (qs > (R)0.0f) w2 = (R)0.5f * minmod(a(C_VV, 1, 0) - a(C_VO, 0, 0), a(C_VV, 0, 0) - a(C_VO, -1, 0));
             if (qs < (R)0.0f) w2 = (R)-0.5f * minmod(a(C_VO, 1, 0) - a(C_VV, 0, 0), a(C_VO, 2, 0) - a(C_VV, 1, 0));
@@ -498,19 +504,26 @@ __device__ __forceinline__ void b_flow_corr(const Dev<R>& S, const Konst<R>& K, 
     if (inside) { hum_c = ld(S.f[HUM] + i); hvm_c = ld(S.f[HVM] + i); }
     if (xrow) hvm_x = ld(S.f[HVM] + i - nx);
     if (xcol) hum_x = ld(S.f[HUM] + IDX(bx0 - 1, by0 + (int)threadIdx.x));
+    const R zref = deep_level<R>(clk);
+    bool deep;
     {
         const R* src[C_NF] = {S.f[ZS], S.f[ZB], S.tmp[T_UU], S.tmp[T_VV], S.f[UUOLD], S.f[VVOLD], S.f[QX], S.f[QY]};
-        tile_load<R, FC_H, C_NF>(tile, src, bx0, by0, nx, ny);
+        deep = tile_load<R, FC_H, true>(tile, src, bx0, by0, nx, ny, zref, deep_bed(K, zref));
     }
-    for (int e = threadIdx.x + threadIdx.y * FT_X; e < FT_N; e += FT_X * FT_Y) {
-        int gx, gy;
-        int k = tile_centre<FC_H>(e % FT_TX + FC_H - 1, e / FT_TX + FC_H - 1, bx0, by0, nx, ny, gx, gy);
-        TileAt<R, FC_H> a{tile, k};
-        R w1, w2, v1, v2;
-        wrk_u(a, K, gx, gy, w1, w2);
-        wrk_v(a, K, gx, gy, v1, v2);
-        sU1[e] = w1; sU2[e] = w2; sV1[e] = v1; sV2[e] = v2;
-    }
+    auto ring = [&](auto dp) {
+        constexpr bool DEEP = decltype(dp)::value;
+        for (int e = threadIdx.x + threadIdx.y * FT_X; e < FT_N; e += FT_X * FT_Y) {
+            int gx, gy;
+            int k = tile_centre<FC_H>(e % FT_TX + FC_H - 1, e / FT_TX + FC_H - 1, bx0, by0, nx, ny, gx, gy);
+            TileAt<R, FC_H> a{tile, k};
+            R w1, w2, v1, v2;
+            wrk_u<R, DEEP>(a, K, gx, gy, w1, w2);
+            wrk_v<R, DEEP>(a, K, gx, gy, v1, v2);
+            sU1[e] = w1; sU2[e] = w2; sV1[e] = v1; sV2[e] = v2;
+        }
+    };
+    if (deep) ring(std::true_type{});
+    else ring(std::false_type{});
     __syncthreads();
     R dtf = (R)clk->dt, rdx = K.rdx;
     const int kc = (threadIdx.y + FC_H) * G::TX + threadIdx.x + FC_H;
@@ -610,15 +623,13 @@ __device__ __forceinline__ void wrk_z(const A& a, const Konst<R>& K, int ix, int
     const R eps2 = K.eps * (R)2.0f;
     w1 = (R)0.0f; w2 = (R)0.0f;
     if (ix > 0) {
-        const Pair2<R> m1 = zz_min<R>(a, -1, 2, 0, 0);   // x-1 .. x+2
-        if (m1.a + m1.b > eps2) {
+        if (zz_deeper<R>(a, -1, 2, 0, 0, eps2)) {   // x-1 .. x+2
             R u = a(Z_UU, 0, 0);
             if (u > (R)0.0f) w1 = u * (R)0.5f * minmod(a(Z_ZS, 1, 0) - a(Z_ZO, 0, 0), a(Z_ZS, 0, 0) - a(Z_ZO, -1, 0));
             if (u < (R)0.0f) w1 = (R)-1.0f * u * (R)0.5f * minmod(a(Z_ZO, 2, 0) - a(Z_ZS, 1, 0), a(Z_ZO, 1, 0) - a(Z_ZS, 0, 0));
         }
         if (iy > 0) {
-            const Pair2<R> m2 = zz_min<R>(a, 0, 0, -1, 2);   // y-1 .. y+2
-            if (m2.a + m2.b > eps2) {
+            if (zz_deeper<R>(a, 0, 0, -1, 2, eps2)) {   // y-1 .. y+2
                 R v = a(Z_VV, 0, 0);
                 if (v > (R)0.0f) w2 = v * (R)0.5f * minmod(a(Z_ZS, 0, 1) - a(Z_ZO, 0, 0), a(Z_ZS, 0, 0) - a(Z_ZO, 0, -1));
                 if (v < (R)0.0f) w2 = v * (R)0.5f * minmod(a(Z_ZO, 0, 2) - a(Z_ZS, 0, 1), a(Z_ZO, 0, 1) - a(Z_ZS, 0, 0));
@@ -685,7 +696,7 @@ __device__ __forceinline__ void b_flow_final(const Dev<R>& S, const Konst<R>& K,
     const int bx0 = bix * FT_X, by0 = biy * FT_Y;
     {
         const R* src[Z_NF] = {S.tmp[T_ZS], S.f[ZB], zsold_in, S.f[UU], S.f[VV], S.f[UST], S.f[THM]};
-        tile_load<R, FC_H, Z_NF>(tile, src, bx0, by0, nx, ny);
+        tile_load<R, FC_H, false>(tile, src, bx0, by0, nx, ny, (R)0, (R)0);
     }
     for (int e = threadIdx.x + threadIdx.y * FT_X; e < FT_N; e += FT_X * FT_Y) {
         int gx, gy;

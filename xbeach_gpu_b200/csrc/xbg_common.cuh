@@ -215,9 +215,12 @@ struct TileG {
 // block.  Fields 0 and 1 (the water level and the bed in every staged pass,
 // read together by the wet tests) are interleaved, t[2 e + f], so a tile
 // cell's pair is one 8-byte (16-byte) shared-memory load; field f >= 2 is
-// the plane t[f * N + e].
-template <class R, int H, int NF>
-__device__ __forceinline__ void tile_load(R* t, const R* const (&src)[NF], int bx0, int by0, int nx, int ny) {
+// the plane t[f * N + e].  With CHECK, returns whether every level of the tile
+// is at least zref and every bed at least bref (each thread looks at what it
+// copied; the barrier that ends the load combines the answers).
+template <class R, int H, bool CHECK, int NF>
+__device__ __forceinline__ bool tile_load(R* t, const R* const (&src)[NF], int bx0, int by0, int nx, int ny, R zref,
+                                          R bref) {
     using G = TileG<H>;
     const int tid = threadIdx.x + threadIdx.y * G::X;
     for (int e = tid; e < G::N; e += G::X * G::Y) {
@@ -230,7 +233,13 @@ __device__ __forceinline__ void tile_load(R* t, const R* const (&src)[NF], int b
     }
     cp_async_commit();
     cp_async_wait_all();
-    __syncthreads();
+    if (!CHECK) {
+        __syncthreads();
+        return false;
+    }
+    bool above = true;
+    for (int e = tid; e < G::N; e += G::X * G::Y) above = above && t[2 * e] >= zref && t[2 * e + 1] >= bref;
+    return __syncthreads_and(above) != 0;
 }
 template <class R> struct Pair2 { R a, b; };
 template <class R> struct alignas(2 * sizeof(R)) Pair2A { R a, b; };
@@ -287,6 +296,19 @@ __device__ __forceinline__ Pair2<R> zz_min(const A& a, int x0, int x1, int y0, i
             m.b = DM<R>::fmin(m.b, v.b);
         }
     return m;
+}
+
+// The second-order corrections apply where min(level) + min(bed) over a window
+// exceeds 2 eps.  A block whose tile has every level above zref and every bed
+// above 2 eps - zref (with a margin far above rounding) passes that test in all
+// its windows, so it skips the minima: zref is a metre below the offshore
+// level, which leaves the minima to the blocks in less than about a metre of
+// water.
+template <class R>
+__device__ __forceinline__ R deep_level(const Clock* clk) { return (R)clk->zsbndi - (R)1; }
+template <class R>
+__device__ __forceinline__ R deep_bed(const Konst<R>& K, R zref) {
+    return K.eps * (R)2.0f - zref + (R)0.01 + DM<R>::fabs(zref) * (R)1e-4;
 }
 
 // Row segments: a thread takes V consecutive cells of one row (V = 4 in
