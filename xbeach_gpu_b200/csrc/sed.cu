@@ -312,129 +312,197 @@ __device__ __forceinline__ void zbl_xy(int ix, int iy, int nx, int ny, int& sx, 
     if (ix == 0) { sx = pp(ix, nx); sy = iy; }
 }
 
-// avalanching (Sediment_kernel.cu:1020-1137) transfers (dzbx, dzby) of (ix, iy)
+// avalanching (Sediment_kernel.cu:1020-1137): the transfer between a cell (bed
+// Zi, sediment thickness si) and its right or upper neighbour (Zn, sn); dzmax:
+// the cell's critical slope
 template <class R>
-__device__ __forceinline__ void aval_cell(const Dev<R>& S, const Konst<R>& K, int ix, int iy, R dtf, R& dzbx, R& dzby) {
-    const int nx = K.nx, ny = K.ny;
-    const R* zb = S.tmp[T_ZB]; const R* sd = S.tmp[T_STDEP];
-    int xp = pp(ix, nx), yp = pp(iy, ny);
-    R Zbi = ld(zb + zbl_src(ix, iy, nx, ny)), Zbt = ld(zb + zbl_src(ix, yp, nx, ny)), Zbr = ld(zb + zbl_src(xp, iy, nx, ny));
-    R sti = ld(sd + zbl_src(ix, iy, nx, ny)), stt = ld(sd + zbl_src(ix, yp, nx, ny)), str = ld(sd + zbl_src(xp, iy, nx, ny));
-    R dx = K.dx, maxchg = K.maxslpchg;
-    R dzmax = ld(S.tmp[T_HH] + IDX(ix, iy)) > K.eps ? K.wetdzmax : K.drydzmax;
-    dzbx = (R)0.0f; dzby = (R)0.0f;
-    R dzbdx = (Zbr - Zbi) / dx;
-    if (DM<R>::fabs(dzbdx) > dzmax) {
-        R s = dzbdx / DM<R>::fabs(dzbdx);
-        dzbx = s * (DM<R>::fabs(dzbdx) - dzmax) * dx;
+__device__ __forceinline__ R aval_of(const Konst<R>& K, R Zi, R Zn, R si, R sn, R dzmax, R dtf) {
+    const R dx = K.dx, maxchg = K.maxslpchg;
+    const R slope = (Zn - Zi) / dx;
+    R d = (R)0.0f;
+    if (DM<R>::fabs(slope) > dzmax) {
+        const R s = slope / DM<R>::fabs(slope);
+        d = s * (DM<R>::fabs(slope) - dzmax) * dx;
         if (s > (R)0) {
-            dzbx = DM<R>::fmin(dzbx, maxchg * dtf / dx);
-            dzbx = DM<R>::fmin(dzbx, sti);
+            d = DM<R>::fmin(d, maxchg * dtf / dx);
+            d = DM<R>::fmin(d, si);
         } else {
-            dzbx = DM<R>::fmax(dzbx, (R)-1.0f * maxchg * dtf / dx);
-            dzbx = DM<R>::fmax(dzbx, (R)-1.0f * str);
+            d = DM<R>::fmax(d, (R)-1.0f * maxchg * dtf / dx);
+            d = DM<R>::fmax(d, (R)-1.0f * sn);
         }
     }
-    R dzbdy = (Zbt - Zbi) / dx;
-    if (DM<R>::fabs(dzbdy) > dzmax) {
-        R s = dzbdy / DM<R>::fabs(dzbdy);
-        dzby = s * (DM<R>::fabs(dzbdy) - dzmax) * dx;
-        if (s > (R)0) {
-            dzby = DM<R>::fmin(dzby, maxchg * dtf / dx);
-            dzby = DM<R>::fmin(dzby, sti);
-        } else {
-            dzby = DM<R>::fmax(dzby, (R)-1 * maxchg * dtf / dx);
-            dzby = DM<R>::fmax(dzby, (R)-1 * stt);
-        }
-    }
+    return d;
 }
-
-// bed change of (ix, iy) gathered from its own and its neighbours' transfers,
-// in the order a serial launch adds them: ((-dzby[below] - dzbx[left]) + dzbx) + dzby
 template <class R>
-__device__ __forceinline__ R ddzb_cell(const Dev<R>& S, const Konst<R>& K, int ix, int iy, R dtf) {
-    R a = (R)0.0f, bx, by, t;
-    if (iy > 0) { aval_cell(S, K, ix, iy - 1, dtf, t, by); a = a - by; }
-    if (ix > 0) { aval_cell(S, K, ix - 1, iy, dtf, bx, t); a = a - bx; }
-    aval_cell(S, K, ix, iy, dtf, bx, by);
+__device__ __forceinline__ R aval_max(const Konst<R>& K, R hh) { return hh > K.eps ? K.wetdzmax : K.drydzmax; }
+
+// bed change of a cell gathered from its own and its neighbours' transfers, in
+// the order a serial launch adds them: ((-dzby[below] - dzbx[left]) + dzbx) + dzby
+template <class R>
+__device__ __forceinline__ R ddzb_of(int ix, int iy, R by_below, R bx_left, R bx, R by) {
+    R a = (R)0.0f;
+    if (iy > 0) a = a - by_below;
+    if (ix > 0) a = a - bx_left;
     a = a + bx;
     a = a + by;
     return a;
 }
 
-// zblatbnd, avalanching, updatezb, zblatbnd, updatezom.  The transfers
-// (dzbx, dzby) of every cell of the 32 x 8 tile, the column to its left and
-// the row below it go to shared memory once; a boundary cell whose zblatbnd
-// source lies elsewhere evaluates that source's bed change directly.
+// ... of cell (ix, iy), everything from global memory: the beds and
+// thicknesses are those after zblatbnd (zbl_src)
+template <class R>
+__device__ __forceinline__ R ddzb_cell(const Dev<R>& S, const Konst<R>& K, int ix, int iy, R dtf) {
+    const int nx = K.nx, ny = K.ny;
+    auto zb = [&](int x, int y) { return ld(S.tmp[T_ZB] + zbl_src(x, y, nx, ny)); };
+    auto sd = [&](int x, int y) { return ld(S.tmp[T_STDEP] + zbl_src(x, y, nx, ny)); };
+    const int xm = mm(ix), xp = pp(ix, nx), ym = mm(iy), yp = pp(iy, ny);
+    const R* hh = S.tmp[T_HH];
+    const R z = zb(ix, iy), zl = zb(xm, iy), zr = zb(xp, iy), zd = zb(ix, ym), zu = zb(ix, yp);
+    const R t = sd(ix, iy), tl = sd(xm, iy), tr = sd(xp, iy), td = sd(ix, ym), tu = sd(ix, yp);
+    const R h = ld(hh + IDX(ix, iy)), hl = ld(hh + IDX(xm, iy)), hd = ld(hh + IDX(ix, ym));
+    return ddzb_of(ix, iy, aval_of(K, zd, z, td, t, aval_max(K, hd), dtf),
+                   aval_of(K, zl, z, tl, t, aval_max(K, hl), dtf), aval_of(K, z, zr, t, tr, aval_max(K, h), dtf),
+                   aval_of(K, z, zu, t, tu, aval_max(K, h), dtf));
+}
+
+// zb, stdep of a cell: updatezb at its zblatbnd source, then the copy
+// (zblatbnd); zb1, sd1: the source's values before, ds its bed change.
+// updatezom (:1162-1190) gives the friction factors.
+template <class R>
+struct SedC { R zb, sd, cf, fw; };
+template <class R>
+__device__ __forceinline__ SedC<R> sed_c_of(const Konst<R>& K, R zb1, R sd1, R ds) {
+    SedC<R> o;
+    o.zb = zb1 + ds;
+    o.sd = sd1 - ds;
+    const bool reef = o.sd < (R)0.05f;
+    o.cf = reef ? K.cfreef : K.cfsand;
+    o.fw = reef ? K.fwreef : K.fwsand;
+    return o;
+}
+// ... of a boundary cell, whose source lies elsewhere
+template <class R>
+__device__ SedC<R> sed_c_boundary(const Dev<R>& S, const Konst<R>& K, int ix, int iy, R dtf) {
+    int sx, sy;
+    zbl_xy(ix, iy, K.nx, K.ny, sx, sy);
+    const int j = zbl_src(sx, sy, K.nx, K.ny);
+    return sed_c_of(K, ld(S.tmp[T_ZB] + j), ld(S.tmp[T_STDEP] + j), ddzb_cell(S, K, sx, sy, dtf));
+}
+
+// zblatbnd, avalanching, updatezb, zblatbnd, updatezom.  A cell's bed change
+// needs four transfers, its own two and one of each of the cells left and below,
+// from ten beds and thicknesses and three depths around it: every thread loads
+// them and evaluates the four, one round trip to memory and no barrier (with the
+// transfers of the block's tile and a ring shared in shared memory, two round
+// trips and a barrier, the pass took 56 us at 2048 x 1024).
 template <class R>
 __device__ __forceinline__ void b_sed_c(const Dev<R>& S, const Konst<R>& K, const int bix, const int biy) {
     const Clock* clk = S.clk;
-    if (sed_skip(clk)) return;
-    __shared__ R sBx[SB_TY * SB_TX], sBy[SB_TY * SB_TX];
+    const bool off = sed_skip(clk);
     const int nx = K.nx, ny = K.ny;
-    const int bx0 = bix * SB_X, by0 = biy * SB_Y;
+    const int ix = bix * blockDim.x + threadIdx.x, iy = biy * blockDim.y + threadIdx.y;
+    if (ix >= nx || iy >= ny) return;
     const bool morph = K.morfac > (R)0.0f;
     const R dtf = (R)clk->dt;
-    const int ix = bx0 + threadIdx.x, iy = by0 + threadIdx.y;
-    const bool cell = ix < nx && iy < ny;
     const int i = IDX(ix, iy);
-    // the cell's own inputs first, so that their round trip overlaps the tile's
-    R cnew = (R)0, dzb0 = (R)0, zs0 = (R)0, hh0 = (R)0, zb1 = (R)0, sd1 = (R)0;
-    int sx = ix, sy = iy;
-    if (cell) {
-        cnew = ld(S.tmp[T_UU] + i);
-        if (morph) {
-            dzb0 = ld(S.f[DZB] + i);
-            zs0 = ld(S.f[ZS] + i);
-            hh0 = ld(S.tmp[T_HH] + i);
-            zbl_xy(ix, iy, nx, ny, sx, sy);
-            int s1x, s1y;
-            zbl_xy(sx, sy, nx, ny, s1x, s1y);
-            zb1 = ld(S.tmp[T_ZB] + IDX(s1x, s1y));
-            sd1 = ld(S.tmp[T_STDEP] + IDX(s1x, s1y));
-        }
+    const R cnew = ld(S.tmp[T_UU] + i);
+    if (!morph) {
+        loads_before_here();
+        if (!off) S.f[CSED][i] = cnew;
+        return;
     }
-    if (morph) {
-        for (int e = threadIdx.x + threadIdx.y * SB_X; e < SB_TY * SB_TX; e += SB_X * SB_Y) {
-            int gx = min(max(bx0 - 1 + e % SB_TX, 0), nx - 1), gy = min(max(by0 - 1 + e / SB_TX, 0), ny - 1);
-            R a, b;
-            aval_cell(S, K, gx, gy, dtf, a, b);
-            sBx[e] = a;
-            sBy[e] = b;
-        }
-    }
-    __syncthreads();
-    if (!cell) return;
+    const R dzb0 = ld(S.f[DZB] + i), zs0 = ld(S.f[ZS] + i), hh0 = ld(S.tmp[T_HH] + i);
+    const R dd = ddzb_cell(S, K, ix, iy, dtf);
+    const bool edge = ix == 0 || iy == 0 || iy == ny - 1;
+    const SedC<R> o = edge ? sed_c_boundary(S, K, ix, iy, dtf)
+                           : sed_c_of(K, ld(S.tmp[T_ZB] + i), ld(S.tmp[T_STDEP] + i), dd);
+    loads_before_here();
+    if (off) return;
     S.f[CSED][i] = cnew;
-    if (morph) {
-        // bed change gathered in the serial launch order:
-        // ((-dzby[below] - dzbx[left]) + dzbx) + dzby
-        const int c = (threadIdx.y + 1) * SB_TX + threadIdx.x + 1;
-        R dd = (R)0.0f;
-        if (iy > 0) dd = dd - sBy[c - SB_TX];
-        if (ix > 0) dd = dd - sBx[c - 1];
-        dd = dd + sBx[c];
-        dd = dd + sBy[c];
-        // updatezb (:1139-1160) at the own cell
-        S.f[DZB][i] = dzb0 - dd;
-        S.f[ZS][i] = zs0 - dd;
-        S.f[HH][i] = hh0 - dd;
-        // zb, stdep: updatezb at the zblatbnd source, then the copy
-        const int s = IDX(sx, sy);
-        R ds = (s == i) ? dd : ddzb_cell(S, K, sx, sy, dtf);
-        R zbn = zb1 + ds;
-        R sdn = sd1 - ds;
-        S.f[ZB][i] = zbn;
-        S.f[STDEP][i] = sdn;
-        // updatezom (:1162-1190)
-        if (sdn < (R)0.05f) { S.f[CFM][i] = K.cfreef; S.f[FWM][i] = K.fwreef; }
-        else { S.f[CFM][i] = K.cfsand; S.f[FWM][i] = K.fwsand; }
-    }
+    // updatezb (:1139-1160) at the own cell
+    S.f[DZB][i] = dzb0 - dd;
+    S.f[ZS][i] = zs0 - dd;
+    S.f[HH][i] = hh0 - dd;
+    S.f[ZB][i] = o.zb;
+    S.f[STDEP][i] = o.sd;
+    S.f[CFM][i] = o.cf;
+    S.f[FWM][i] = o.fw;
 }
 XBG_KERNELS(sed_c)
 
-// wide: the pointwise first pass in 64 x 4 blocks instead of 32 x 8; vec: over
-// row segments (where nx is a multiple of the segment width)
+// The same pass over row segments (Seg), with the same arithmetic.
+template <class R>
+__global__ void __launch_bounds__(256) k_sed_c_v(Dev<R> S, Konst<R> K) {
+    using G = Seg<R>;
+    using U = typename G::U;
+    constexpr int V = G::V;
+    const Clock* clk = S.clk;
+    const bool off = sed_skip(clk);
+    const int nx = K.nx, ny = K.ny;
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (iy >= ny) return;   // the whole warp: a warp is one row
+    const G g(nx, blockIdx.x);
+    const bool morph = K.morfac > (R)0.0f;
+    const R dtf = (R)clk->dt;
+    const U cnew = g.row(S.tmp[T_UU], iy);
+    if (!morph) {
+        loads_before_here();
+        if (!off && g.act) g.put(S.f[CSED], iy, cnew);
+        return;
+    }
+    // a row of zb or stdep after zblatbnd: rows 0 and ny-1 are rows 1 and ny-2,
+    // column 0 is the row's own column 1
+    auto src = [&](int y) { return y == 0 ? 1 : (y == ny - 1 ? ny - 2 : y); };
+    auto row = [&](const R* f, int y) {
+        U u = g.row(f, src(y));
+        if (g.x0 == 0) u.a[0] = src(y) == y ? u.a[1] : ld(f + 1 + (size_t)y * nx);
+        return u;
+    };
+    const int ym = mm(iy), yp = pp(iy, ny);
+    const R* zb = S.tmp[T_ZB]; const R* sd = S.tmp[T_STDEP];
+    const U z = row(zb, iy), zd = row(zb, ym), zu = row(zb, yp), t = row(sd, iy), td = row(sd, ym), tu = row(sd, yp),
+            h = g.row(S.tmp[T_HH], iy), hd = g.row(S.tmp[T_HH], ym), dzb0 = g.row(S.f[DZB], iy),
+            zs0 = g.row(S.f[ZS], iy);
+    const R zl = g.left(z, zb, src(iy)), zr = g.right(z, zb, src(iy)), tl = g.left(t, sd, src(iy)),
+            tr = g.right(t, sd, src(iy)), hl = g.left(h, S.tmp[T_HH], iy);
+    U o_dzb, o_zs, o_hh, o_zb, o_sd, o_cf, o_fw;
+    R left = aval_of(K, zl, z.a[0], tl, t.a[0], aval_max(K, hl), dtf);   // dzbx of the cell left of k
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const R hm = aval_max(K, h.a[k]);
+        const R bx = aval_of(K, z.a[k], k < V - 1 ? z.a[k + 1] : zr, t.a[k], k < V - 1 ? t.a[k + 1] : tr, hm, dtf);
+        const R by = aval_of(K, z.a[k], zu.a[k], t.a[k], tu.a[k], hm, dtf);
+        const R below = aval_of(K, zd.a[k], z.a[k], td.a[k], t.a[k], aval_max(K, hd.a[k]), dtf);
+        const R dd = ddzb_of(g.x0 + k, iy, below, left, bx, by);
+        left = bx;
+        const SedC<R> o = sed_c_of(K, z.a[k], t.a[k], dd);
+        o_dzb.a[k] = dzb0.a[k] - dd; o_zs.a[k] = zs0.a[k] - dd; o_hh.a[k] = h.a[k] - dd;
+        o_zb.a[k] = o.zb; o_sd.a[k] = o.sd; o_cf.a[k] = o.cf; o_fw.a[k] = o.fw;
+    }
+    if (!g.act) return;
+    if (iy == 0 || iy == ny - 1 || g.x0 == 0) {   // boundary cells
+#pragma unroll
+        for (int k = 0; k < V; k++) {
+            if (k > 0 && iy != 0 && iy != ny - 1) break;
+            const SedC<R> o = sed_c_boundary(S, K, g.x0 + k, iy, dtf);
+            o_zb.a[k] = o.zb; o_sd.a[k] = o.sd; o_cf.a[k] = o.cf; o_fw.a[k] = o.fw;
+        }
+    }
+    loads_before_here();
+    if (off) return;
+    g.put(S.f[CSED], iy, cnew);
+    g.put(S.f[DZB], iy, o_dzb);
+    g.put(S.f[ZS], iy, o_zs);
+    g.put(S.f[HH], iy, o_hh);
+    g.put(S.f[ZB], iy, o_zb);
+    g.put(S.f[STDEP], iy, o_sd);
+    g.put(S.f[CFM], iy, o_cf);
+    g.put(S.f[FWM], iy, o_fw);
+}
+
+// wide: the pointwise first pass in 64 x 4 blocks instead of 32 x 8; vec: the
+// first and third pass over row segments (where nx is a multiple of the segment
+// width)
 template <class R>
 int launch_sed(const Dev<R>& S, const Konst<R>& K, cudaStream_t st, Prof* pf, bool wide, bool vec) {
     dim3 b(32, 8), g((K.nx + 31) / 32, (K.ny + 7) / 8);
@@ -445,7 +513,8 @@ int launch_sed(const Dev<R>& S, const Konst<R>& K, cudaStream_t st, Prof* pf, bo
     PMARK(pf, "k_sed_a");
     k_sed_b<R><<<g, b, 0, st>>>(S, K);
     PMARK(pf, "k_sed_b");
-    k_sed_c<R><<<g, b, 0, st>>>(S, K);
+    if (vec && K.nx % V == 0) k_sed_c_v<R><<<dim3((K.nx / V + 31) / 32, (K.ny + 7) / 8), b, 0, st>>>(S, K);
+    else k_sed_c<R><<<g, b, 0, st>>>(S, K);
     PMARK(pf, "k_sed_c");
     return 3;
 }
