@@ -11,7 +11,7 @@
 //                units), then energint, roelvink|baldock, dissipation,
 //                meandir, radstress.  Each bin's ee/rr plane tile (32 x 8
 //                cells + 2-cell halo) streams into shared memory by cp.async
-//                three bins ahead (five buffers, one barrier per bin), and
+//                several bins ahead (one barrier per bin), and
 //                the cell's own bins for the theta fluxes come from the
 //                resident tiles; ctheta
 //                (propagtheta) is evaluated on the fly from per-cell slopes;
@@ -96,8 +96,7 @@ __device__ __forceinline__ CthCoef<R> cth_coef(const Dev<R>& S, const Konst<R>& 
     c.dvdy = (ld(vv + ix + yp * nx) - ld(vv + ix + ym * nx)) / sy;
     int i = ix + iy * nx;
     R h = ld(hh + i);
-    R kh = cmin(ld(S.f[WK] + i) * h, (R)10.0f);
-    c.s = sg / DM<R>::sinh((R)2.0f * kh);
+    c.s = ld(S.tmp[T_SIG] + i);   // sigma / sinh(2 kh), from the dispersion pass
     c.wci = K.wci * cmin(h / K.hwci, (R)1.0f);
     c.sg = sg;
     return c;
@@ -348,20 +347,25 @@ __device__ __forceinline__ R wave_edge_cell(const Dev<R>& S, const Konst<R>& K, 
 
 // Plane tile buffers.  At bin t planes t, t+1 and t+2 are resident (the
 // stencil of plane t; the cell's own values of planes t+1 and t+2 for the
-// theta fluxes) and plane t+3 streams in; it goes into the buffer of plane
-// t-2, which every thread finished reading before the previous barrier.
-constexpr int WT_NB = 5;
+// theta fluxes), WT_LEAD planes are in flight and the last of them goes into
+// the buffer of plane t-2, which every thread finished reading before the
+// previous barrier.  In FP32 three planes: with one, every bin waited for its
+// copies' latency (768 x 384 x 12 bins with currents 65 us).  In FP64 one, which
+// leaves shared memory for two blocks per SM.
+template <class R> constexpr int WT_LEAD = sizeof(R) == 4 ? 3 : 1;
+template <class R> constexpr int WT_NB = 4 + WT_LEAD<R>;
 
 template <class R, bool ROLLER, bool WCI>
 __device__ __forceinline__ void b_wave_fast(const Dev<R>& S, const Konst<R>& K, const int bix, const int biy) {
+    constexpr int NB = WT_NB<R>, LEAD = WT_LEAD<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Clock* clk = S.clk;
     if (wave_off(clk)) return;
     const int nx = K.nx, ny = K.ny, nt = K.nt, C = S.C;
     const int tid = threadIdx.x + threadIdx.y * WT_X;
-    R* tE = (R*)smem_raw;                 // [WT_NB][WT_N] plane tiles of ee
-    R* tR = tE + WT_NB * WT_N;            // [WT_NB][WT_N] plane tiles of rr
-    R* sA = tR + WT_NB * WT_N;            // [nt][256] advected ee (energy units)
+    R* tE = (R*)smem_raw;                 // [NB][WT_N] plane tiles of ee
+    R* tR = tE + NB * WT_N;            // [NB][WT_N] plane tiles of rr
+    R* sA = tR + NB * WT_N;            // [nt][256] advected ee (energy units)
     R* sR = sA + (size_t)nt * 256;        // [nt][256] advected rr
     Dir4<R>* sMom = reinterpret_cast<Dir4<R>*>(sR + (size_t)nt * 256);   // [nt]
     Dir2<R>* sCS2 = reinterpret_cast<Dir2<R>*>(sMom + nt);               // [nt]
@@ -440,10 +444,9 @@ __device__ __forceinline__ void b_wave_fast(const Dev<R>& S, const Konst<R>& K, 
         const R ctht = DM<R>::fma(cthP, sx, cthQ * cx);
         return cmin(cmax(ctht, (R)(-0.25f * cc.sg)), (R)(0.25f * cc.sg));
     };
-    // planes 0, 1, 2 (empty groups past the last plane)
-    issue(0);
-    if (nt > 1) issue(1); else cp_async_commit();
-    if (nt > 2) issue(2); else cp_async_commit();
+    // planes 0 .. LEAD + 1 (empty groups past the last plane)
+    for (int k = 0; k < LEAD + 2; k++)
+        if (k < nt) issue(k); else cp_async_commit();
     __syncthreads();   // theta tables
     if (active) {
         i = ix + iy * nx;
@@ -472,7 +475,7 @@ __device__ __forceinline__ void b_wave_fast(const Dev<R>& S, const Konst<R>& K, 
         c0 = cth(sCS2[0].c, sCS2[0].s);
         cpp = cth(sCS2[cl(1)].c, sCS2[cl(1)].s);
     }
-    cp_async_wait1();   // planes 0 and 1 have landed (this thread's copies)
+    cp_async_wait<LEAD>();   // planes 0 and 1 have landed (this thread's copies)
     fixup(0);
     if (nt > 1) fixup(1);
     R* oA = sA + tid;
@@ -480,11 +483,11 @@ __device__ __forceinline__ void b_wave_fast(const Dev<R>& S, const Konst<R>& K, 
     const R* oldR = rro + i;   // without the roller pass rr is carried unchanged
 #pragma unroll 1
     for (int t = 0; t < nt; t++) {
-        const int b = t % WT_NB;
-        if (t + 3 < nt) issue((t + 3) % WT_NB);
+        const int b = t % NB;
+        if (t + 2 + LEAD < nt) issue((t + 2 + LEAD) % NB);
         else cp_async_commit();
-        cp_async_wait1();   // plane t+2 has landed (this thread's copies)
-        if (t + 2 < nt) fixup((t + 2) % WT_NB);
+        cp_async_wait<LEAD>();   // plane t+2 has landed (this thread's copies)
+        if (t + 2 < nt) fixup((t + 2) % NB);
         __syncthreads();    // ... and every thread's
         if (active) {
             const R* qE = tE + b * WT_N + ctile;
@@ -495,7 +498,7 @@ __device__ __forceinline__ void b_wave_fast(const Dev<R>& S, const Konst<R>& K, 
                 we2 = qE[0]; we1 = we2; we3 = tE[b1 * WT_N + ctile];
                 if (ROLLER) { wr2 = qR[0]; wr1 = wr2; wr3 = tR[b1 * WT_N + ctile]; }
             }
-            const int b2 = (t + 2 < nt ? t + 2 : nt - 1) % WT_NB;
+            const int b2 = (t + 2 < nt ? t + 2 : nt - 1) % NB;
             we4 = tE[b2 * WT_N + ctile];
             if (ROLLER) wr4 = tR[b2 * WT_N + ctile];
             const Dir2<R> d = sCS2[t];
@@ -629,11 +632,11 @@ __device__ __forceinline__ void b_wave_fast(const Dev<R>& S, const Konst<R>& K, 
     block_min_store<R>(dtw, S.part_wave + bix + biy * ((K.nx + 31) / 32));
 }
 template <class R, bool ROLLER, bool WCI>
-__global__ void __launch_bounds__(256, 3) k_wave_fast(Dev<R> S, Konst<R> K) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_wave_fast(Dev<R> S, Konst<R> K) {
     b_wave_fast<R, ROLLER, WCI>(S, K, blockIdx.x, blockIdx.y);
 }
 template <class R, bool ROLLER, bool WCI>
-__global__ void __launch_bounds__(256, 3) kb_wave_fast(BatchTab<R> T, const int2* items, int n) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) kb_wave_fast(BatchTab<R> T, const int2* items, int n) {
     batch_items<R>(T, items, n, [&](const Dev<R>& S, const Konst<R>& K, const BatchAux&, int bx, int by) {
         b_wave_fast<R, ROLLER, WCI>(S, K, bx, by);
     });
@@ -665,7 +668,7 @@ void launch_wave_fast_batch(const BatchTab<R>& T, const BatchLaunch& L, int roll
     }
 }
 template <class R>
-size_t wave_fast_smem(int nt) { return ((size_t)2 * WT_NB * WT_N + (size_t)2 * nt * 256 + 6 * nt) * sizeof(R); }
+size_t wave_fast_smem(int nt) { return ((size_t)2 * WT_NB<R> * WT_N + (size_t)2 * nt * 256 + 6 * nt) * sizeof(R); }
 
 // ------------------------------------------------------------------------
 // Rows pass with tensor-memory-accelerator (TMA) tiles: the same arithmetic
