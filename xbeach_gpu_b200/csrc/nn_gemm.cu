@@ -23,6 +23,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -1440,6 +1441,257 @@ __global__ void k_wgrad_reduce(const float* __restrict__ part, float* __restrict
     }
 }
 
+// ------------------------------------------------------------------------
+// The weight gradient with box copies (W a multiple of 64, cin of 16, BN <= 128).
+// k_wgrad_tc gathers every 64-pixel chunk of its 128 k columns once per tap,
+// thread by thread, and its threads meet twice per chunk: about a microsecond
+// per chunk whatever it holds.  Here
+//  - a CTA takes WC input channels and the same contiguous run of chunks (64
+//    pixels of an image row) as a CTA of k_wgrad_tc, in the same order, so that
+//    every slice of `part` is equal bit for bit;
+//  - a copy warp streams the run's input chunks, one image row ahead and from one
+//    row behind, each as three boxes shifted by the taps' x offset, and the chunks of
+//    dz; boxes end in zeros beyond the image, which is the padding;
+//  - a product warp adds, for chunk i and each of the taps' y offsets, the
+//    transposed product of input chunk i + dy * nseg (its three boxes stacked
+//    along M; nseg: chunks of an image row) and dz chunk i to one accumulator per
+//    y offset: an input chunk is copied three times instead of nine and serves
+//    three rows of dz while 2 nseg + 1 chunks stay resident;
+//  - the fourth box of a slot holds ones in its first channel, so that one row
+//    of the product is the bias gradient; further rows of the 128 (WC = 16)
+//    multiply what follows the slot and are not stored.
+// Waits as in k_conv_rows.  Against k_wgrad_tc: 32 -> 32 channels at 4 x 256 x
+// 256 pixels 47 -> 36 us, 96 -> 32 there 103 -> 69, 192 -> 64 at 4 x 128 x 128 61
+// -> 40, 128 -> 128 at 4 x 64 x 64 16 -> 12.  Runs down 64-pixel columns, which copy
+// fewer surrounding rows, took 22 us for the first of these, but sum in another order,
+// and Adam's normalised steps carry the last bits of a small gradient into the weights.
+constexpr int WR_P = 64;    // pixels of a chunk
+constexpr int WR_MX = 24;   // input slots at most
+constexpr int WR_ND = 3;    // dz slots
+
+// [B, H, W, ld] channels-last in boxes of WC channels x 64 pixels
+template <int WC>
+bool strip_map(const void* X, int B, int H, int W, int ld, CUtensorMap* m) {
+    PFN_cuTensorMapEncodeTiled_v12000 enc = map_encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)ld, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+    const cuuint64_t strides[3] = {(cuuint64_t)ld * 2, (cuuint64_t)W * ld * 2, (cuuint64_t)H * W * ld * 2};
+    const cuuint32_t box[4] = {(cuuint32_t)WC, (cuuint32_t)WR_P, 1, 1}, es[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(X), dims, strides, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, WC == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+               : WC == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                          : CU_TENSOR_MAP_SWIZZLE_32B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN, int WC>
+__global__ void __launch_bounds__(192, 1)
+    k_wgrad_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap zmap,
+                 float* __restrict__ part, int HS, int nseg, int chunks, int per, int NX, int cin, int ldp,
+                 int bias_row, int* err) {
+    constexpr int WB = BN % 64 == 0 ? 64 : (BN % 32 == 0 ? 32 : 16);   // dz channels of a box
+    constexpr int ND = WR_ND;
+    constexpr unsigned XL = WC == 32 ? 4u : 6u, ZL = WB == 64 ? 2u : (WB == 32 ? 4u : 6u);
+    constexpr unsigned XG = WC * 2 * 8, ZG = WB * 2 * 8;   // bytes of eight pixels
+    constexpr unsigned XB = WR_P * WC * 2, ZB = WR_P * WB * 2;   // bytes of a box
+    constexpr unsigned XS = 4 * XB, ZS = WR_P * BN * 2;    // bytes of a slot
+    constexpr int TCOLS = BN <= 16 ? 64 : (BN <= 32 ? 128 : (BN <= 64 ? 256 : 512));
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long xfull[WR_MX], xempty[WR_MX], zfull[ND], zempty[ND], done;
+    __shared__ unsigned tmem_slot;
+    __shared__ int bad;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c0 = blockIdx.x * WC;
+    const int u0 = min(chunks, (int)blockIdx.y * per), u1 = min(chunks, u0 + per);
+    const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    unsigned char* gbase = smem_raw + (base - smem_u32(smem_raw));
+    const unsigned zbase = base + (unsigned)(NX + (WC == 16)) * XS;
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(TCOLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    // the ones of each slot's fourth box (16-byte pieces in the box's swizzle)
+    for (int e = tid; e < NX * WR_P * (WC / 8); e += 192) {
+        const int slot = e / (WR_P * (WC / 8)), q = e - slot * (WR_P * (WC / 8));
+        const unsigned lin = (unsigned)q * 16;
+        const unsigned at = lin ^ (((lin >> 7) & (WC == 32 ? 3u : 1u)) << 4);
+        *(uint4*)(gbase + slot * XS + 3 * XB + at) = make_uint4(q % (WC / 8) == 0 ? 0x3F80u : 0u, 0u, 0u, 0u);
+    }
+    if (tid == 0) {
+        bad = 0;
+        for (int k = 0; k < NX; k++) { mbar_init(smem_u32(&xfull[k]), 1); mbar_init(smem_u32(&xempty[k]), 1); }
+        for (int k = 0; k < ND; k++) { mbar_init(smem_u32(&zfull[k]), 1); mbar_init(smem_u32(&zempty[k]), 1); }
+        mbar_init(smem_u32(&done), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = tmem_slot;
+    unsigned leader;   // one lane of each warp
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
+    auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
+    if (warp == 0) {   // ---- copies: per image of the run, input chunks i0 - nseg .. i1 - 1 + nseg, dz chunks i0 .. i1 - 1
+        auto box = [&](unsigned dst, const CUtensorMap* m, int c, int x, int y, int b, unsigned bar) {
+            asm volatile(
+                "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+                "%3, %4, %5}], [%6];\n" ::"r"(dst),
+                "l"((unsigned long long)m), "r"(c), "r"(x), "r"(y), "r"(b), "r"(bar)
+                : "memory");
+        };
+        int xs = 0, zs = 0, nxl = 0, nzl = 0;
+        unsigned xp = 0, zp = 0;
+        bool go = true;
+        for (int u = u0; u < u1 && go;) {
+            const int b = u / HS, i0 = u - b * HS, n = min(u1 - u, HS - i0);   // HS: chunks of an image
+            int xsg = i0 % nseg, xy = i0 / nseg - 1, zsg = xsg, zy = xy + 1;
+            for (int r = -nseg; r < n + nseg; r++) {
+                if (!wait(smem_u32(&xempty[xs]), xp ^ 1u)) { go = false; break; }
+                if (leader) {
+                    const unsigned fb = smem_u32(&xfull[xs]), d = base + (unsigned)xs * XS;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"(3 * XB)
+                                 : "memory");
+                    for (int k = 0; k < 3; k++) box(d + k * XB, &xmap, c0, xsg * WR_P + k - 1, xy, b, fb);
+                }
+                nxl++;
+                if (++xs == NX) { xs = 0; xp ^= 1u; }
+                if (++xsg == nseg) { xsg = 0; xy++; }
+                if (r < nseg) continue;   // dz chunk r - nseg with the last input chunk it meets
+                if (!wait(smem_u32(&zempty[zs]), zp ^ 1u)) { go = false; break; }
+                if (leader) {
+                    const unsigned fb = smem_u32(&zfull[zs]), d = zbase + (unsigned)zs * ZS;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"(ZS)
+                                 : "memory");
+                    for (int k = 0; k < BN / WB; k++) box(d + k * ZB, &zmap, k * WB, zsg * WR_P, zy, b, fb);
+                }
+                nzl++;
+                if (++zs == ND) { zs = 0; zp ^= 1u; }
+                if (++zsg == nseg) { zsg = 0; zy++; }
+            }
+            u += n;
+        }
+        if (*(volatile int*)&bad) {   // leaving early: the copies in flight land first (bounded)
+            for (int k = max(nxl - NX, 0); k < nxl; k++) mbar_wait(smem_u32(&xfull[k % NX]), (k / NX) & 1);
+            for (int k = max(nzl - ND, 0); k < nzl; k++) mbar_wait(smem_u32(&zfull[k % ND]), (k / ND) & 1);
+        }
+    } else if (warp == 1) {   // ---- products
+        const uint32_t idesc = idesc_bf16(GM, BN) | (1u << 15) | (1u << 16);   // A and B MN-major
+        auto commit = [&](unsigned long long* bar) {
+            if (leader)
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                                 smem_u32(bar))
+                             : "memory");
+        };
+        auto next = [&](int k) { return k + 1 == NX ? 0 : k + 1; };
+        // xi: the slot of the chunk one row below (its first of three); xw: the next slot to wait for
+        int xi = 0, xw = 0, held = 0, zs = 0, first = 1;
+        unsigned xp = 0, zp = 0;
+        bool go = true;
+        for (int u = u0; u < u1 && go;) {
+            const int n = min(u1 - u, HS - u % HS);
+            for (int r = 0; r < n; r++) {
+                for (; held < 2 * nseg + 1 && go; held++) {   // chunks xi .. xi + 2 nseg have landed
+                    go = wait(smem_u32(&xfull[xw]), xp);
+                    if (++xw == NX) { xw = 0; xp ^= 1u; }
+                }
+                if (go) go = wait(smem_u32(&zfull[zs]), zp);
+                if (!go) break;
+                tc_fence_after();
+                const unsigned z = zbase + (unsigned)zs * ZS;
+                int sl = xi;
+#pragma unroll
+                for (int dy = 0; dy < 3; dy++) {
+                    const unsigned x = base + (unsigned)sl * XS;
+#pragma unroll
+                    for (int j = 0; j < WR_P / 16; j++)
+                        if (leader)
+                            asm volatile(
+                                "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + dy * BN),
+                                "l"(mn_desc(x + j * 2 * XG, XB, XG, XL)), "l"(mn_desc(z + j * 2 * ZG, ZB, ZG, ZL)),
+                                "r"(idesc), "r"(j || !first ? 1u : 0u));
+                    sl += nseg;
+                    if (sl >= NX) sl -= NX;
+                }
+                first = 0;
+                commit(&zempty[zs]);
+                commit(&xempty[xi]);
+                xi = next(xi);
+                held--;
+                if (++zs == ND) { zs = 0; zp ^= 1u; }
+            }
+            if (!go) break;
+            for (; held > 0; held--) {   // the image's last chunks
+                commit(&xempty[xi]);
+                xi = next(xi);
+            }
+            u += n;
+        }
+        commit(&done);   // every product issued so far
+        if (*(volatile int*)&bad) mbar_wait(smem_u32(&done), 0);
+    } else {   // ---- accumulator row m of y offset dy: x offset m / WC, channel m % WC
+        const int q = warp & 3;
+        if (__all_sync(0xffffffffu, wait(smem_u32(&done), 0)) && !*(volatile int*)&bad) {
+            tc_fence_after();
+            const int m = q * 32 + lane, box = m / WC, ch = m - box * WC;
+            float* dst = part + (size_t)blockIdx.y * BN * ldp;
+            if (q * 32 < 4 * WC)   // the whole warp
+#pragma unroll 1
+                for (int dy = 0; dy < 3; dy++) {
+                    const bool bias = box == 3 && ch == 0 && dy == 0 && c0 == 0 && bias_row;
+                    const int k = bias ? 9 * cin : (dy * 3 + box) * cin + c0 + ch;
+                    const bool out = box < 3 || bias;
+#pragma unroll 1
+                    for (int n = 0; n < BN; n += 16) {
+                        unsigned v[16];
+                        load_cols<16>(v, tmem + ((unsigned)(q * 32) << 16) + (unsigned)(dy * BN + n));
+                        if (out)
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                dst[(size_t)(n + j) * ldp + k] = u1 > u0 ? __uint_as_float(v[j]) : 0.0f;
+                    }
+                }
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && bad) atomicExch(err, XBG_ERR_TIMEOUT);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS));
+}
+
+// false where the shape does not fit (*rc unset), else launched with status *rc
+template <int BN, int WC>
+bool wgrad_rows_launch(const void* X, const void* Dz, float* work, int Bn, int H, int W, int cin, int ldx, int ldz,
+                       int ldp, int bias_row, int ksplit, int* err, cudaStream_t st, int* rc) {
+    constexpr int XS = 4 * WR_P * WC * 2, MAXB = 226 * 1024;
+    const int nseg = W / WR_P, chunks = Bn * H * nseg, per = (chunks + ksplit - 1) / ksplit;
+    // the resident chunks and two to four copies ahead; the rows around a run are
+    // copied too, so a run is at least as long as they are
+    const int fixed = 1024 + (WC == 16 ? XS : 0) + WR_ND * WR_P * BN * 2;
+    const int NX = std::min(std::min(2 * nseg + 5, WR_MX), (MAXB - fixed) / XS);
+    if (NX < 2 * nseg + 3 || per < 2 * nseg) return false;
+    CUtensorMap xm, zm;
+    if (!strip_map<WC>(X, Bn, H, W, ldx, &xm) ||
+        !strip_map<(BN % 64 == 0 ? 64 : (BN % 32 == 0 ? 32 : 16))>(Dz, Bn, H, W, ldz, &zm))
+        return false;
+    static bool attr = false;
+    *rc = XBG_ERR_CUDA;
+    if (!attr) {
+        if (cudaFuncSetAttribute(k_wgrad_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAXB) !=
+            cudaSuccess)
+            return true;
+        attr = true;
+    }
+    k_wgrad_rows<BN, WC><<<dim3((unsigned)(cin / WC), (unsigned)ksplit), 192, (size_t)(fixed + NX * XS), st>>>(
+        xm, zm, work, H * nseg, nseg, chunks, per, NX, cin, ldp, bias_row, err);
+    if (cudaGetLastError() == cudaSuccess) *rc = XBG_OK;
+    return true;
+}
+
 template <int BN>
 int wgrad_launch(const void* X, const void* Dz, float* gw, float* gb, float* work, int Bn, int H, int W, int cin,
                  int ldx, int ldz, int ldw, int ksplit, int accumulate, int* err, cudaStream_t st) {
@@ -1455,13 +1707,23 @@ int wgrad_launch(const void* X, const void* Dz, float* gw, float* gb, float* wor
     const int Kc = 9 * cin;
     const int ldp = Kc + 8;
     const int bias_row = gb ? 1 : 0;
-    dim3 grid((unsigned)((Kc + bias_row + GM - 1) / GM), (unsigned)ksplit);
-    k_wgrad_tc<BN><<<grid, 256, smem, st>>>((const __nv_bfloat16*)X, (const __nv_bfloat16*)Dz, work, Bn, H, W, cin,
-                                            ldx, ldz, ldp, bias_row, err);
-    if (cudaGetLastError() != cudaSuccess) return XBG_ERR_CUDA;
+    int rc = XBG_OK;
+    bool rows = false;
+    if constexpr (BN <= 128) {   // box copies where the shape tiles
+        if (g_conv_tma && W % WR_P == 0 && cin % 32 == 0)
+            rows = wgrad_rows_launch<BN, 32>(X, Dz, work, Bn, H, W, cin, ldx, ldz, ldp, bias_row, ksplit, err, st, &rc);
+        else if (g_conv_tma && W % WR_P == 0 && cin % 16 == 0)
+            rows = wgrad_rows_launch<BN, 16>(X, Dz, work, Bn, H, W, cin, ldx, ldz, ldp, bias_row, ksplit, err, st, &rc);
+    }
+    if (rc != XBG_OK) return rc;
+    if (!rows) {
+        dim3 grid((unsigned)((Kc + bias_row + GM - 1) / GM), (unsigned)ksplit);
+        k_wgrad_tc<BN><<<grid, 256, smem, st>>>((const __nv_bfloat16*)X, (const __nv_bfloat16*)Dz, work, Bn, H, W,
+                                                cin, ldx, ldz, ldp, bias_row, err);
+        if (cudaGetLastError() != cudaSuccess) return XBG_ERR_CUDA;
+    }
     k_wgrad_reduce<<<dim3((unsigned)((Kc + bias_row + 127) / 128), BN), dim3(32, 8), 0, st>>>(work, gw, gb, BN, Kc,
-                                                                                             ldp, ldw, ksplit,
-                                                                                             accumulate);
+                                                                                             ldp, ldw, ksplit, accumulate);
     return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA;
 }
 
