@@ -131,6 +131,26 @@ int xbg_nn_mse(const float* pred, const float* tgt, void* dpred, float* loss,
 int xbg_nn_adam(float* p, void* pb, const float* g, float* m, float* v,
                 long long n, float lr, float b1, float b2, float eps, int step,
                 void* stream);
+/* The same over several arrays in one launch: array k is t[k] (n values each, at
+ * most XBG_NN_MANY arrays). */
+#define XBG_NN_MANY 32
+typedef struct {
+    float* p;
+    void* pb;
+    const float* g;
+    float* m;
+    float* v;
+    long long n;
+} xbg_nn_adam_t;
+int xbg_nn_adam_many(const xbg_nn_adam_t* t, int n, float lr, float b1,
+                     float b2, float eps, int step, void* stream);
+/* xbg_nn_conv3x3_flip over several layers (at most XBG_NN_MANY) in one launch. */
+typedef struct {
+    const void* w;
+    void* wf;
+    int ldw, cin, cd, ldf;
+} xbg_nn_flip_t;
+int xbg_nn_conv3x3_flip_many(const xbg_nn_flip_t* t, int n, void* stream);
 int xbg_nn_to_bf16(const float* a, void* b, long long n, void* stream);
 /* dst[c][p] = src[c][p] for nc planes (DEVICE arrays of plane pointers). */
 int xbg_nn_copy_planes(const float* const* src, float* const* dst, int nc,

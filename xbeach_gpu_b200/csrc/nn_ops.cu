@@ -319,18 +319,37 @@ __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ 
 
 // Adam on fp32 master weights p (n values), keeping a bf16 copy pb (same
 // layout) for the GEMMs; lr_t is the bias-corrected step size.
-__global__ void k_adam(float* __restrict__ p, bf* __restrict__ pb, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, long long n, float lr_t, float b1, float b2, float eps, float vcorr) {
-    long long i = (long long)blockIdx.x * TPB + threadIdx.x;
-    if (i >= n) return;
-    float gi = g[i];
-    float mi = b1 * m[i] + (1.0f - b1) * gi;
-    float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    float pi = p[i] - lr_t * mi / (sqrtf(vi * vcorr) + eps);
-    p[i] = pi;
-    pb[i] = __float2bfloat16(pi);
+struct AdamStep { float lr_t, b1, b2, eps, vcorr; };
+__device__ __forceinline__ void adam_one(const xbg_nn_adam_t& t, const AdamStep& a, long long i) {
+    float gi = t.g[i];
+    float mi = a.b1 * t.m[i] + (1.0f - a.b1) * gi;
+    float vi = a.b2 * t.v[i] + (1.0f - a.b2) * gi * gi;
+    t.m[i] = mi;
+    t.v[i] = vi;
+    float pi = t.p[i] - a.lr_t * mi / (sqrtf(vi * a.vcorr) + a.eps);
+    t.p[i] = pi;
+    ((bf*)t.pb)[i] = __float2bfloat16(pi);
+}
+__global__ void k_adam(xbg_nn_adam_t t, AdamStep a) {
+    const long long i = (long long)blockIdx.x * TPB + threadIdx.x;
+    if (i < t.n) adam_one(t, a, i);
+}
+
+// Several arrays in one launch: a block finds its array by the running block
+// count `first`.  A network's arrays one by one are launches of 2.7 us each
+// whatever they hold (30 of them 82 us; in one 18).
+struct Many { unsigned first[XBG_NN_MANY + 1]; };
+struct AdamMany { xbg_nn_adam_t t[XBG_NN_MANY]; Many b; };
+struct FlipMany { xbg_nn_flip_t t[XBG_NN_MANY]; Many b; };
+__device__ __forceinline__ int many_of(const Many& b) {
+    int k = 0;
+    while (blockIdx.x >= b.first[k + 1]) k++;
+    return k;
+}
+__global__ void k_adam_many(const __grid_constant__ AdamMany A, AdamStep a) {
+    const int k = many_of(A.b);
+    const long long i = (long long)(blockIdx.x - A.b.first[k]) * TPB + threadIdx.x;
+    if (i < A.t[k].n) adam_one(A.t[k], a, i);
 }
 
 // f32 -> bf16 (n values) and bf16 -> f32
@@ -429,16 +448,20 @@ __global__ void k_copy_planes(const float* const* __restrict__ src, float* const
 using namespace xbg::nn;
 
 // wf[c][tap*cd + n] = w[n][(8-tap)*cin + c]; zero for k >= 9*cd
-__global__ void k_flip3x3(const bf* __restrict__ w, int ldw, int cin, int cd, bf* __restrict__ wf, int ldf) {
-    const long long idx = (long long)blockIdx.x * TPB + threadIdx.x;
-    if (idx >= (long long)cin * ldf) return;
-    const int c = (int)(idx / ldf), k = (int)(idx - (long long)c * ldf);
+__device__ __forceinline__ void flip_one(const xbg_nn_flip_t& t, long long idx) {
+    if (idx >= (long long)t.cin * t.ldf) return;
+    const int c = (int)(idx / t.ldf), k = (int)(idx - (long long)c * t.ldf);
     bf v = __float2bfloat16(0.0f);
-    if (k < 9 * cd) {
-        const int tap = k / cd, n = k - tap * cd;
-        v = w[(size_t)n * ldw + (8 - tap) * cin + c];
+    if (k < 9 * t.cd) {
+        const int tap = k / t.cd, n = k - tap * t.cd;
+        v = ((const bf*)t.w)[(size_t)n * t.ldw + (8 - tap) * t.cin + c];
     }
-    wf[idx] = v;
+    ((bf*)t.wf)[idx] = v;
+}
+__global__ void k_flip3x3(xbg_nn_flip_t t) { flip_one(t, (long long)blockIdx.x * TPB + threadIdx.x); }
+__global__ void k_flip3x3_many(const __grid_constant__ FlipMany F) {
+    const int k = many_of(F.b);
+    flip_one(F.t[k], (long long)(blockIdx.x - F.b.first[k]) * TPB + threadIdx.x);
 }
 
 // dst[b][r][q] = src[s_b][y_b + r][x_b + q] for crop x crop pixels of `wpp`
@@ -458,6 +481,10 @@ __global__ void k_gather_crops(const unsigned* __restrict__ src, unsigned* __res
 }
 
 #define NN_LAUNCH(n) if ((n) <= 0) return XBG_OK; cudaStream_t st_ = (cudaStream_t)stream
+static AdamStep adam_step(float lr, float b1, float b2, float eps, int step) {
+    const float bc1 = 1.0f - powf(b1, (float)step), bc2 = 1.0f - powf(b2, (float)step);
+    return AdamStep{lr / bc1, b1, b2, eps, 1.0f / bc2};
+}
 #define NN_DONE return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA
 
 extern "C" {
@@ -481,7 +508,23 @@ int xbg_nn_conv3x3_flip(const void* w, int ldw, int cin, int cd, void* wf, int l
     if (!w || !wf || cin < 1 || cd < 1 || ldw < 9 * cin || ldf < 9 * cd) return XBG_ERR_ARG;
     long long n = (long long)cin * ldf;
     NN_LAUNCH(n);
-    k_flip3x3<<<blocks_for(n), TPB, 0, st_>>>((const bf*)w, ldw, cin, cd, (bf*)wf, ldf);
+    k_flip3x3<<<blocks_for(n), TPB, 0, st_>>>(xbg_nn_flip_t{w, wf, ldw, cin, cd, ldf});
+    NN_DONE;
+}
+int xbg_nn_conv3x3_flip_many(const xbg_nn_flip_t* t, int n, void* stream) {
+    if (!t || n < 0 || n > XBG_NN_MANY) return XBG_ERR_ARG;
+    FlipMany F{};
+    long long blocks = 0;
+    for (int k = 0; k < n; k++) {
+        if (!t[k].w || !t[k].wf || t[k].cin < 1 || t[k].cd < 1 || t[k].ldw < 9 * t[k].cin || t[k].ldf < 9 * t[k].cd)
+            return XBG_ERR_ARG;
+        F.t[k] = t[k];
+        blocks += ((long long)t[k].cin * t[k].ldf + TPB - 1) / TPB;
+        if (blocks > 0x7fffffffLL) return XBG_ERR_ARG;
+        F.b.first[k + 1] = (unsigned)blocks;
+    }
+    NN_LAUNCH(blocks);
+    k_flip3x3_many<<<(unsigned)blocks, TPB, 0, st_>>>(F);
     NN_DONE;
 }
 int xbg_nn_gather_crops(const void* src, void* dst, const int* idx, int B, int ny, int nx, int crop,
@@ -571,8 +614,22 @@ int xbg_nn_adam(float* p, void* pb, const float* g, float* m, float* v, long lon
                 float eps, int step, void* stream) {
     if (!p || !pb || !g || !m || !v || n < 0 || step < 1) return XBG_ERR_ARG;
     NN_LAUNCH(n);
-    float bc1 = 1.0f - powf(b1, (float)step), bc2 = 1.0f - powf(b2, (float)step);
-    k_adam<<<blocks_for(n), TPB, 0, st_>>>(p, (bf*)pb, g, m, v, n, lr / bc1, b1, b2, eps, 1.0f / bc2);
+    k_adam<<<blocks_for(n), TPB, 0, st_>>>(xbg_nn_adam_t{p, pb, g, m, v, n}, adam_step(lr, b1, b2, eps, step));
+    NN_DONE;
+}
+int xbg_nn_adam_many(const xbg_nn_adam_t* t, int n, float lr, float b1, float b2, float eps, int step, void* stream) {
+    if (!t || n < 0 || n > XBG_NN_MANY || step < 1) return XBG_ERR_ARG;
+    AdamMany A{};
+    long long blocks = 0;
+    for (int k = 0; k < n; k++) {
+        if (!t[k].p || !t[k].pb || !t[k].g || !t[k].m || !t[k].v || t[k].n < 0) return XBG_ERR_ARG;
+        A.t[k] = t[k];
+        blocks += (t[k].n + TPB - 1) / TPB;
+        if (blocks > 0x7fffffffLL) return XBG_ERR_ARG;
+        A.b.first[k + 1] = (unsigned)blocks;
+    }
+    NN_LAUNCH(blocks);
+    k_adam_many<<<(unsigned)blocks, TPB, 0, st_>>>(A, adam_step(lr, b1, b2, eps, step));
     NN_DONE;
 }
 int xbg_nn_encode(const float* const* planes, int nc, const float* mean, const float* inv_std, void* x, long long P,

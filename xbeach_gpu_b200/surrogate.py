@@ -120,6 +120,14 @@ def _np_for(cout):
     raise ValueError(cout)
 
 
+class _AdamArray(C.Structure):   # xbg_nn_adam_t
+    _fields_ = [(n, C.c_void_p) for n in ("p", "pb", "g", "m", "v")] + [("n", C.c_longlong)]
+
+
+class _FlipLayer(C.Structure):   # xbg_nn_flip_t
+    _fields_ = [("w", C.c_void_p), ("wf", C.c_void_p)] + [(n, C.c_int) for n in ("ldw", "cin", "cd", "ldf")]
+
+
 def _bind_ops(L):
     vp, ip, ll, fl = C.c_void_p, C.c_int, C.c_longlong, C.c_float
     L.xbg_nn_im2col3x3.argtypes = [vp, vp, ip, ip, ip, ip, ip, ip, vp]
@@ -136,6 +144,8 @@ def _bind_ops(L):
     L.xbg_nn_chan_copy.argtypes = [vp, vp, ll, ip, ip, ip, ip, ip, vp]
     L.xbg_nn_mse.argtypes = [vp, vp, vp, vp, ip, ip, ip, ip, vp]
     L.xbg_nn_adam.argtypes = [vp, vp, vp, vp, vp, ll, fl, fl, fl, fl, ip, vp]
+    L.xbg_nn_adam_many.argtypes = [C.POINTER(_AdamArray), ip, fl, fl, fl, fl, ip, vp]
+    L.xbg_nn_conv3x3_flip_many.argtypes = [C.POINTER(_FlipLayer), ip, vp]
     L.xbg_nn_to_bf16.argtypes = [vp, vp, ll, vp]
     L.xbg_nn_encode.argtypes = [vp, ip, vp, vp, vp, ll, vp]
     L.xbg_nn_decode.argtypes = [vp, ip, vp, vp, vp, vp, ip, ll, vp]
@@ -207,6 +217,10 @@ class Conv3x3:
         been used)."""
         L = lib()
         _ok(L.xbg_nn_conv3x3_flip(_p(self.wb), self.Kp, self.cin, self.Np, _p(self.wf), self.Kd, None), "flip W")
+        self.refresh_wt()
+
+    def refresh_wt(self):
+        L = lib()
         if self.wt is not None:
             _ok(L.xbg_nn_transpose(_p(self.wb), _p(self.wt), self.Np, self.Kp, self.Kp, self.Nk, None),
                 "transpose W")
@@ -472,11 +486,14 @@ class UNet:
     def adam(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.nstep += 1
         L = lib()
-        for l in self.L.values():
-            for (p_, pb, g, m, v) in l.params():
-                _ok(L.xbg_nn_adam(_p(p_), _p(pb), _p(g), _p(m), _p(v), p_.numel(), lr, b1, b2, eps, self.nstep,
-                                  None), "adam")
-            l.refresh_t()
+        layers = list(self.L.values())
+        arrays = [(*(t.data_ptr() for t in a), a[0].numel()) for l in layers for a in l.params()]
+        _ok(L.xbg_nn_adam_many((_AdamArray * len(arrays))(*arrays), len(arrays), lr, b1, b2, eps, self.nstep, None),
+            "adam")
+        flips = [(l.wb.data_ptr(), l.wf.data_ptr(), l.Kp, l.cin, l.Np, l.Kd) for l in layers]
+        _ok(L.xbg_nn_conv3x3_flip_many((_FlipLayer * len(flips))(*flips), len(flips), None), "flip W")
+        for l in layers:
+            l.refresh_wt()
 
     def train_step(self, x, tgt, B, H, W, lr=1e-3):
         """One Adam step on a batch; returns the loss (device scalar).  The
