@@ -38,8 +38,7 @@ template <class R>
 __device__ void wavebnd_cursor(Clock& c, const Konst<R>& K, const Series* ser);
 
 template <class R>
-__device__ void finalize_scalar(const Dev<R>& S, const Konst<R>& K, const Series* ser, R mflow, R mwave) {
-    Clock& c = *S.clk;
+__device__ void finalize_scalar(Clock& c, const Konst<R>& K, const Series* ser, R mflow, R mwave) {
     c.halt = 1;
     if (c.status != XBG_OK) return;
     if (c.flags & (XBG_FLAG_OUTPUT_DUE | XBG_FLAG_ENDED)) return;
@@ -81,7 +80,12 @@ __device__ __forceinline__ void b_step_begin(const Dev<R>& S, const Konst<R>& K,
                                              int nwave, const int bi, const int nb) {
     __shared__ R red[8], rw[8];
     __shared__ int last;
+    // the clock, read with the fields: the last block's scalar pass would otherwise
+    // wait for one dependent load after another
+    constexpr int CW = (int)(sizeof(Clock) / 8);
+    __shared__ unsigned long long sclk[CW];
     int tid = threadIdx.x;
+    if (tid < CW) sclk[tid] = ((const volatile unsigned long long*)S.clk)[tid];
     R m = (R)3.0e38f;
     {   // FLOWDT: max of hh first (16-byte loads, two of each field in flight
         // per thread), one sqrt per thread
@@ -168,8 +172,10 @@ __device__ __forceinline__ void b_step_begin(const Dev<R>& S, const Konst<R>& K,
     if (tid == 0) {
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) { mf = DM<R>::fmin(mf, red[w]); mw = DM<R>::fmin(mw, rw[w]); }
         *S.counter = 0;
-        finalize_scalar(S, K, ser, mf, mw);
+        finalize_scalar(*reinterpret_cast<Clock*>(sclk), K, ser, mf, mw);
     }
+    __syncthreads();
+    if (tid < CW) ((unsigned long long*)S.clk)[tid] = sclk[tid];
 }
 template <class R>
 __global__ void __launch_bounds__(256) k_step_begin(Dev<R> S, Konst<R> K, const Series* ser, int nflow, int nwave) {
