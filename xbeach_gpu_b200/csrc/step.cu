@@ -246,15 +246,22 @@ __device__ __forceinline__ void b_ubnd(const Dev<R>& S, const Konst<R>& K, const
     Clock* clk = S.clk;
     if (halted(clk)) return;
     const int nx = K.nx, ny = K.ny;
-    if (threadIdx.x == 0) {   // flowbnd sea level and wind (Wave_gpu.cu:1020-1103)
+    // flowbnd sea level and wind (Wave_gpu.cu:1020-1103), a warp each: both are
+    // chains of dependent loads and divisions
+    const int wind = nthr > 32 ? 32 : 0;
+    if (threadIdx.x == 0) {
         Clock& c = *clk;
-        double t = c.totaltime;
+        const double t = c.totaltime;
         advance_cursor(ser->slt, c.nsl, c.SLstep, t);
         int s = c.SLstep;
         c.zsbndi = interptime(ser->sla[s], ser->sla[s - 1], ser->slt[s] - ser->slt[s - 1], t - ser->slt[s - 1]);
         c.zsbndn = interptime(ser->slb[s], ser->slb[s - 1], ser->slt[s] - ser->slt[s - 1], t - ser->slt[s - 1]);
+    }
+    if ((int)threadIdx.x == wind) {
+        Clock& c = *clk;
+        const double t = c.totaltime;
         advance_cursor(ser->wt, c.nwnd, c.WNDstep, t);
-        s = c.WNDstep;
+        const int s = c.WNDstep;
         c.windu = (double)(R)interptime(ser->wa[s], ser->wa[s - 1], ser->wt[s] - ser->wt[s - 1], t - ser->wt[s - 1]);
         c.windv = (double)(R)interptime(ser->wb[s], ser->wb[s - 1], ser->wt[s] - ser->wt[s - 1], t - ser->wt[s - 1]);
     }
