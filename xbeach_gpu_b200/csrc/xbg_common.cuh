@@ -430,18 +430,21 @@ __device__ __forceinline__ void batch_items(const BatchTab<R>& T, const int2* it
 }
 
 // Single-domain and batched kernels of a 256-thread body b_NAME(S, K, bx, by).
-#define XBG_BATCH_KERNEL(NAME)                                                                         \
+// XBG_KERNELS_B: the FP32 batched kernel with room for MIN resident blocks (the
+// scenario's table in shared memory costs the bodies registers); 0 leaves the
+// compiler's choice
+#define XBG_KERNELS_B(NAME, MIN)                                                                       \
     template <class R>                                                                                 \
-    __global__ void __launch_bounds__(256) kb_##NAME(BatchTab<R> T, const int2* items, int n) {        \
+    __global__ void __launch_bounds__(256, sizeof(R) == 4 ? MIN : 0)                                   \
+        kb_##NAME(BatchTab<R> T, const int2* items, int n) {                                           \
         batch_items<R>(T, items, n, [&](const Dev<R>& S, const Konst<R>& K, const BatchAux&, int bx,   \
                                         int by) { b_##NAME<R>(S, K, bx, by); });                       \
-    }
-#define XBG_KERNELS(NAME)                                                                              \
+    }                                                                                                  \
     template <class R>                                                                                 \
     __global__ void __launch_bounds__(256) k_##NAME(Dev<R> S, Konst<R> K) {                            \
         b_##NAME<R>(S, K, blockIdx.x, blockIdx.y);                                                     \
-    }                                                                                                  \
-    XBG_BATCH_KERNEL(NAME)
+    }
+#define XBG_KERNELS(NAME) XBG_KERNELS_B(NAME, 0)
 
 // Early exit of a kernel in a step that the device clock has halted.  The
 // flow passes, the second sediment pass and the dispersion pass read the
