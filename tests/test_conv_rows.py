@@ -14,6 +14,8 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(1, 1, 128, 16, 16), (1, 5, 128, 32, 32), (3, 37, 128, 32, 48), (2, 64, 256, 64, 64), (1, 211, 384, 96, 32),
           (2, 33, 256, 32, 96), (1, 300, 128, 64, 128), (1, 64, 1024, 16, 32), (5, 67, 128, 48, 64),
           (1, 32, 256, 32, 128),
+          # ragged last strips: one pixel short, one over a strip and a half, rows too narrow for strips
+          (1, 40, 255, 32, 32), (2, 21, 193, 16, 64), (1, 70, 344, 64, 64), (3, 5, 1000, 96, 32), (1, 9, 129, 32, 48),
           # tile by tile: rows of 64, 32, 16 pixels; many and few tiles
           (1, 16, 64, 64, 64), (2, 32, 32, 128, 256), (4, 16, 16, 384, 128), (1, 130, 128, 256, 192),
           (2, 128, 128, 128, 128), (1, 64, 128, 256, 256), (3, 64, 128, 192, 64)]

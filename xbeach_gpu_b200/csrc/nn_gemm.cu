@@ -634,11 +634,12 @@ inline PFN_cuTensorMapEncodeTiled_v12000 map_encoder() {
     }
     return enc;
 }
+// (ragged: in boxes of 128 pixels of one row, W at least that, the last one beyond the image)
 template <int WC>
-bool conv_map(const void* X, int B, int H, int W, int cin, int ldx, CUtensorMap* m) {
+bool conv_map(const void* X, int B, int H, int W, int cin, int ldx, CUtensorMap* m, bool ragged = false) {
     if (cin % WC || ldx % 8) return false;
     const int Wt = W >= GM ? GM : W;
-    if (W >= GM ? (W % GM) : (GM % W)) return false;
+    if (ragged ? W < GM : (W >= GM ? (W % GM) : (GM % W))) return false;
     const int R = GM / Wt;
     if (H % R) return false;
     PFN_cuTensorMapEncodeTiled_v12000 enc = map_encoder();
@@ -727,7 +728,8 @@ __device__ __forceinline__ void store_cols(unsigned taddr, const float* bias, vo
 
 // ------------------------------------------------------------------------
 // The forward convolution over rows of 128 pixels, for layers whose weights
-// fit in shared memory beside the input stages (W a multiple of 128, N <= 128).
+// fit in shared memory beside the input stages (N <= 128; the last strip of a
+// width that is no multiple of 128 ends in zeros and is stored in part).
 // k_conv_tma loads an output tile's input nine times, once per tap, and starts
 // and drains a pipeline for every 128 pixels: its time is the copies' latency.
 // Here
@@ -775,7 +777,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
     __shared__ int bad;
     __shared__ float sbias[BN];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int strips = W / GM, total = Bn * strips * H, ncg = cin / WC, nb = 3 * ncg;   // boxes of an input row
+    const int strips = (W + GM - 1) / GM, total = Bn * strips * H, ncg = cin / WC, nb = 3 * ncg;   // boxes of an input row
     const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x;
     const int lo = (int)blockIdx.x * per, hi = min(total, lo + per);
     if (lo >= hi) return;   // the whole CTA
@@ -943,7 +945,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
                             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(&aempty[slot]))
                                          : "memory");
                     }
-                    put_cols<CW>(v, sbias + c0, Y, row * ldy + c0, flags);
+                    if (x0 + q * 32 + lane < W) put_cols<CW>(v, sbias + c0, Y, row * ldy + c0, flags);
                 }
             }
             return true;
@@ -959,7 +961,9 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
 // stages that fit beside the weights of a layer (0: k_conv_rows does not apply)
 template <int BN, int WC>
 int conv_rows_stages(int W, int cin) {
-    if (BN > 128 || W % GM) return 0;
+    // the last strip of a row may be ragged; strips of which over a third lies outside the image are not worth it
+    const int strips = (W + GM - 1) / GM;
+    if (BN > 128 || W < GM || 2 * strips * GM > 3 * W) return 0;
     const int room = 225 * 1024 - 1024 - 9 * cin * BN * 2, box = GM * WC * 2;
     const int n = room < 0 ? 0 : room / box;
     const int nb = 3 * (cin / WC);   // an input row's boxes are waited for together; two rows' worth, or nearly
@@ -979,7 +983,7 @@ int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, vo
             return XBG_ERR_CUDA;
         sms = n;
     }
-    const long long total = (long long)Bn * (W / GM) * H;
+    const long long total = (long long)Bn * ((W + GM - 1) / GM) * H;
     const size_t smem = 1024 + (size_t)nst * GM * WC * 2 + (size_t)9 * cin * BN * 2;
     k_conv_rows<BN, WC><<<(unsigned)(total < sms ? total : sms), CR_THREADS, smem, st>>>(
         m, (const __nv_bfloat16*)Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err);
@@ -1164,37 +1168,34 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
         attr = true;
     }
     const long long M = (long long)Bn * H * W;
-    if (g_conv_tma && M % GM == 0) {   // box copies of the input when the shape tiles
-        // over rows where the weights fit beside the stages (the input is read
-        // three times instead of nine), else tile by tile in 64-channel chunks,
-        // else (channel counts that are no multiple of 64) k_conv_tma
-        CUtensorMap m;
-        if constexpr (BN <= 128) {
-            if (cin % 64 == 0) {
-                const int nst = conv_rows_stages<BN, 64>(W, cin);
-                if (nst && conv_map<64>(X, Bn, H, W, cin, ldx, &m))
-                    return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
-            }
+    CUtensorMap m;
+    if constexpr (BN <= 128) {
+        // over rows where the weights fit beside the stages (the input is read three
+        // times instead of nine)
+        if (g_conv_tma) {
+            int nst = 0;
+            if (cin % 64 == 0 && (nst = conv_rows_stages<BN, 64>(W, cin)) &&
+                conv_map<64>(X, Bn, H, W, cin, ldx, &m, true))
+                return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
+            if (cin % 32 == 0 && (nst = conv_rows_stages<BN, 32>(W, cin)) &&
+                conv_map<32>(X, Bn, H, W, cin, ldx, &m, true))
+                return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
+            if (cin % 32 != 0 && cin % 16 == 0 && (nst = conv_rows_stages<BN, 16>(W, cin)) &&
+                conv_map<16>(X, Bn, H, W, cin, ldx, &m, true))
+                return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
         }
+    }
+    if (g_conv_tma && M % GM == 0) {   // box copies of the input when the shape tiles
+        // tile by tile in 64-channel chunks, else (channel counts that are no
+        // multiple of 64) k_conv_tma
         if constexpr (BN % 64 == 0) {
-            if (cin % 64 == 0 && !(BN <= 128 && conv_rows_stages<(BN <= 128 ? BN : 128), 32>(W, cin)) &&
-                conv_map<64>(X, Bn, H, W, cin, ldx, &m))
+            if (cin % 64 == 0 && conv_map<64>(X, Bn, H, W, cin, ldx, &m))
                 return conv_ws(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
         }
-        if (cin % 32 == 0 && conv_map<32>(X, Bn, H, W, cin, ldx, &m)) {
-            if constexpr (BN <= 128) {
-                const int nst = conv_rows_stages<BN, 32>(W, cin);
-                if (nst) return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
-            }
+        if (cin % 32 == 0 && conv_map<32>(X, Bn, H, W, cin, ldx, &m))
             return conv_tma_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
-        }
-        if (cin % 32 != 0 && conv_map<16>(X, Bn, H, W, cin, ldx, &m)) {
-            if constexpr (BN <= 128) {
-                const int nst = conv_rows_stages<BN, 16>(W, cin);
-                if (nst) return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
-            }
+        if (cin % 32 != 0 && conv_map<16>(X, Bn, H, W, cin, ldx, &m))
             return conv_tma_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
-        }
     }
     k_conv_tc<BN><<<(unsigned)((M + GM - 1) / GM), 256, smem, st>>>((const __nv_bfloat16*)X,
                                                                      (const __nv_bfloat16*)Wt, bias, Y, Bn, H, W, cin,
