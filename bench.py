@@ -33,7 +33,7 @@ B_ALGO = lambda nt: 4 * (77 + 4 * nt)   # algorithmic bytes per coupled cell-upd
 # (kernel, nx, ny, ntheta); other workloads report traffic null.
 NCU_TRAFFIC = {
     ("k_wave_fast", 2048, 1024, 18): 361049088 + 335545344,
-    ("k_wave_tma", 2048, 1024, 18): 345307392 + 328110592,
+    ("k_wave_tma", 2048, 1024, 18): 354084608 + 332685568,
 }
 
 

@@ -1072,7 +1072,7 @@ __device__ __forceinline__ double clamp_nan(double v, double lo, double hi) { re
 // about 2.4 us to land under load whatever the box (108 to 187 cycles per box
 // and SM in a pure stream of boxes of 1 to 7 KB), and the arithmetic of a bin
 // runs beside the other blocks' waits only.  At 2048 x 1024 x 18 bins the pass
-// takes 283 us (2.6 TB/s of its 352 bytes per cell); without any x, y, theta
+// takes 277 us (2.7 TB/s of its 352 bytes per cell); without any x, y, theta
 // and dissipation arithmetic it takes 190.  One cell per thread, four buffers
 // and boxes with halos on both sides took 334 us.
 //  1. Advection, V neighbouring cells of a row per thread.  One wide
@@ -1386,8 +1386,8 @@ __device__ __forceinline__ void b_wave_tma(const Dev<R>& S, const Konst<R>& K, c
 // (128 threads, 111 registers, four blocks per SM by shared memory at 18 bins);
 // four cells of one field on as many threads take 306 against 285 us at
 // 2048 x 1024, four cells of both on 64 threads leave too few warps (332 us).
-// FP64: two cells (16-byte loads at most) of one field on 256 threads (71
-// against 79 us at 512 x 256 for both fields on 128).  Without the roller a
+// FP64: two cells (16-byte loads at most) of one field on 256 threads (66
+// against 74 us at 512 x 256 for both fields on 128).  Without the roller a
 // thread has four (FP64: two) cells.
 template <class R, bool ROLLER> constexpr bool wave_split = ROLLER && sizeof(R) == 8;
 template <class R, bool ROLLER> constexpr int wave_v = sizeof(R) == 8 || ROLLER ? 2 : 4;
