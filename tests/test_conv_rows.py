@@ -18,7 +18,9 @@ SHAPES = [(1, 1, 128, 16, 16), (1, 5, 128, 32, 32), (3, 37, 128, 32, 48), (2, 64
           (1, 40, 255, 32, 32), (2, 21, 193, 16, 64), (1, 70, 344, 64, 64), (3, 5, 1000, 96, 32), (1, 9, 129, 32, 48),
           # tile by tile: rows of 64, 32, 16 pixels; many and few tiles
           (1, 16, 64, 64, 64), (2, 32, 32, 128, 256), (4, 16, 16, 384, 128), (1, 130, 128, 256, 192),
-          (2, 128, 128, 128, 128), (1, 64, 128, 256, 256), (3, 64, 128, 192, 64)]
+          (2, 128, 128, 128, 128), (1, 64, 128, 256, 256), (3, 64, 128, 192, 64),
+          # ragged tiles: last rows, last columns, rows of 43, 100 and 7 pixels
+          (1, 65, 43, 256, 128), (2, 31, 100, 128, 64), (1, 50, 7, 64, 192), (2, 9, 172, 384, 128), (1, 33, 316, 192, 64)]
 
 
 @pytest.mark.parametrize("f32,relu", [(False, True), (True, False)])

@@ -634,14 +634,14 @@ inline PFN_cuTensorMapEncodeTiled_v12000 map_encoder() {
     }
     return enc;
 }
-// (ragged: in boxes of 128 pixels of one row, W at least that, the last one beyond the image)
+// (ragged: boxes at the right and lower edge may reach beyond the image)
 template <int WC>
 bool conv_map(const void* X, int B, int H, int W, int cin, int ldx, CUtensorMap* m, bool ragged = false) {
     if (cin % WC || ldx % 8) return false;
     const int Wt = W >= GM ? GM : W;
-    if (ragged ? W < GM : (W >= GM ? (W % GM) : (GM % W))) return false;
+    if (!ragged && (W >= GM ? (W % GM) : (GM % W))) return false;
     const int R = GM / Wt;
-    if (H % R) return false;
+    if (ragged ? H < R : H % R) return false;
     PFN_cuTensorMapEncodeTiled_v12000 enc = map_encoder();
     if (!enc) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)ldx, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
@@ -992,7 +992,8 @@ int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, vo
 
 // ------------------------------------------------------------------------
 // The forward convolution as k_conv_tma (the same products in the same order,
-// an output tile of 128 pixels x BN of the layer's channels per CTA) with a warp
+// an output tile of up to 128 pixels, whole rows or part of one, the last ones of
+// an image ragged, x BN of the layer's channels per CTA) with a warp
 // for the copies, one for the products and four for the tile's store, for
 // inputs of a multiple of 64 channels.  k_conv_tma's threads meet twice per
 // 64-wide chunk and its next copies wait for the last chunk's products, so a
@@ -1002,6 +1003,8 @@ int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, vo
 // and one of the weights ([BN][64]).  Waits as in k_conv_rows.  Against
 // k_conv_tma: 256 -> 256 channels at 64 x 128 pixels 50 -> 14 us, 384 -> 128 at
 // 128 x 256 69 -> 27, 192 -> 64 at 256 x 512 94 -> 47.
+// With ragged tiles (and strips in k_conv_rows) instead of the gathered path, a
+// prediction of 240 x 1016 pixels takes 328 instead of 623 us, of 128 x 200 221 of 346.
 template <int BN, int ST>
 __global__ void __launch_bounds__(192, 1)
     k_conv_ws(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
@@ -1012,7 +1015,10 @@ __global__ void __launch_bounds__(192, 1)
     __shared__ unsigned tmem_slot;
     __shared__ int bad;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * GM, n0 = blockIdx.y * BN, nk = 9 * cin / GK;
+    // the tile: R rows of Wt pixels from (x0, y0) of image b
+    const int Wt = min(W, GM), R = GM / Wt, tx = (W + Wt - 1) / Wt, ty = (H + R - 1) / R;
+    const int b = blockIdx.x / (tx * ty), y0 = (int)blockIdx.x / tx % ty * R, x0 = (int)blockIdx.x % tx * Wt;
+    const int n0 = blockIdx.y * BN, nk = 9 * cin / GK;
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
@@ -1033,14 +1039,14 @@ __global__ void __launch_bounds__(192, 1)
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
     auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
     if (warp == 0) {   // ---- copies
-        const int HW = H * W, b = m0 / HW, rem = m0 - b * HW, y0 = rem / W, x0 = rem - y0 * W;
+        const unsigned bytes = (unsigned)(R * Wt) * GK * 2 + B_BYTES;
         int s = 0, c0 = 0, dx = -1, dy = -1, kc = 0;
         unsigned ph = 0;
         for (; kc < nk; kc++) {
             if (!wait(smem_u32(&empty[s]), ph ^ 1u)) break;
             if (leader) {
                 const unsigned fb = smem_u32(&full[s]), sa = base + (unsigned)s * STAGE;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"((unsigned)STAGE)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"(bytes)
                              : "memory");
                 asm volatile(
                     "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
@@ -1094,11 +1100,15 @@ __global__ void __launch_bounds__(192, 1)
         const int q = warp & 3;
         if (__all_sync(0xffffffffu, wait(smem_u32(&done), 0)) && !*(volatile int*)&bad) {
             tc_fence_after();
-            const size_t row = (size_t)m0 + q * 32 + lane;
+            const int p = q * 32 + lane, r = p / Wt, x = x0 + p - r * Wt, y = y0 + r;
+            const size_t row = (size_t)(b * H + y) * W + x;
+            const bool inside = r < R && x < W && y < H;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32)
-                store_cols<32>(tmem + ((unsigned)(q * 32) << 16) + (unsigned)c0, bias ? bias + n0 + c0 : nullptr, Y,
-                               row * ldy + n0 + c0, flags);
+            for (int c0 = 0; c0 < BN; c0 += 32) {
+                unsigned v[32];
+                load_cols<32>(v, tmem + ((unsigned)(q * 32) << 16) + (unsigned)c0);
+                if (inside) put_cols<32>(v, bias ? bias + n0 + c0 : nullptr, Y, row * ldy + n0 + c0, flags);
+            }
         }
     }
     __syncthreads();
@@ -1119,6 +1129,11 @@ inline bool weight_map(const void* Wt, int rows, int Kp, int ldw, int bn, CUtens
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+inline long long conv_ws_tiles(int Bn, int H, int W) {
+    const int Wt = W < GM ? W : GM, R = GM / Wt;
+    return (long long)Bn * ((W + Wt - 1) / Wt) * ((H + R - 1) / R);
+}
+
 template <int BN, int ST>
 int conv_ws_launch(const CUtensorMap& xm, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
                    int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
@@ -1132,7 +1147,7 @@ int conv_ws_launch(const CUtensorMap& xm, const void* Wt, const float* bias, voi
     }
     CUtensorMap wm;
     if (!weight_map(Wt, N, Kp, ldw, BN, &wm)) return XBG_ERR_CUDA;
-    const dim3 grid((unsigned)((long long)Bn * H * W / GM), (unsigned)(N / BN));
+    const dim3 grid((unsigned)conv_ws_tiles(Bn, H, W), (unsigned)(N / BN));
     k_conv_ws<BN, ST><<<grid, 192, smem, st>>>(xm, wm, bias, Y, Bn, H, W, cin, ldy, flags, err);
     return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA;
 }
@@ -1142,7 +1157,7 @@ int conv_ws_launch(const CUtensorMap& xm, const void* Wt, const float* bias, voi
 // deep stages where the grid has no second wave, two with half of them elsewhere.
 inline int conv_ws(const CUtensorMap& xm, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
                    int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
-    const long long tiles = (long long)Bn * H * W / GM;
+    const long long tiles = conv_ws_tiles(Bn, H, W);
     const bool wide = N % 128 == 0 && tiles * (N / 128) >= 100;
     const bool deep = tiles * (N / (wide ? 128 : 64)) <= 148;
 #define XBG_CONV_WS(BN, ST) \
@@ -1185,13 +1200,13 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
                 return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
         }
     }
+    // tile by tile in 64-channel chunks where the tiles lie inside the image for two thirds
+    if constexpr (BN % 64 == 0) {
+        if (g_conv_tma && cin % 64 == 0 && 2 * GM * conv_ws_tiles(Bn, H, W) <= 3 * M &&
+            conv_map<64>(X, Bn, H, W, cin, ldx, &m, true))
+            return conv_ws(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
+    }
     if (g_conv_tma && M % GM == 0) {   // box copies of the input when the shape tiles
-        // tile by tile in 64-channel chunks, else (channel counts that are no
-        // multiple of 64) k_conv_tma
-        if constexpr (BN % 64 == 0) {
-            if (cin % 64 == 0 && conv_map<64>(X, Bn, H, W, cin, ldx, &m))
-                return conv_ws(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
-        }
         if (cin % 32 == 0 && conv_map<32>(X, Bn, H, W, cin, ldx, &m))
             return conv_tma_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
         if (cin % 32 != 0 && conv_map<16>(X, Bn, H, W, cin, ldx, &m))
