@@ -11,7 +11,7 @@
 //                units), then energint, roelvink|baldock, dissipation,
 //                meandir, radstress.  Each bin's ee/rr plane tile (32 x 8
 //                cells + 2-cell halo) streams into shared memory by cp.async
-//                several bins ahead (one barrier per bin), and
+//                three bins ahead (five buffers, one barrier per bin), and
 //                the cell's own bins for the theta fluxes come from the
 //                resident tiles; ctheta
 //                (propagtheta) is evaluated on the fly from per-cell slopes;
@@ -347,17 +347,16 @@ __device__ __forceinline__ R wave_edge_cell(const Dev<R>& S, const Konst<R>& K, 
 
 // Plane tile buffers.  At bin t planes t, t+1 and t+2 are resident (the
 // stencil of plane t; the cell's own values of planes t+1 and t+2 for the
-// theta fluxes), WT_LEAD planes are in flight and the last of them goes into
-// the buffer of plane t-2, which every thread finished reading before the
-// previous barrier.  In FP32 three planes: with one, every bin waited for its
-// copies' latency (768 x 384 x 12 bins with currents 65 us).  In FP64 one, which
-// leaves shared memory for two blocks per SM.
-template <class R> constexpr int WT_LEAD = sizeof(R) == 4 ? 3 : 1;
-template <class R> constexpr int WT_NB = 4 + WT_LEAD<R>;
+// theta fluxes) and plane t+3 streams in; it goes into the buffer of plane
+// t-2, which every thread finished reading before the previous barrier.  More
+// planes in flight did not help: with three, 1203 x 599 x 12 bins 121 against 118
+// us and 1001 x 401 x 18 102 against 98; 768 x 384 x 12 with currents the same.
+constexpr int WT_LEAD = 1;
+constexpr int WT_NB = 4 + WT_LEAD;
 
 template <class R, bool ROLLER, bool WCI>
 __device__ __forceinline__ void b_wave_fast(const Dev<R>& S, const Konst<R>& K, const int bix, const int biy) {
-    constexpr int NB = WT_NB<R>, LEAD = WT_LEAD<R>;
+    constexpr int NB = WT_NB, LEAD = WT_LEAD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Clock* clk = S.clk;
     if (wave_off(clk)) return;
@@ -668,7 +667,7 @@ void launch_wave_fast_batch(const BatchTab<R>& T, const BatchLaunch& L, int roll
     }
 }
 template <class R>
-size_t wave_fast_smem(int nt) { return ((size_t)2 * WT_NB<R> * WT_N + (size_t)2 * nt * 256 + 6 * nt) * sizeof(R); }
+size_t wave_fast_smem(int nt) { return ((size_t)2 * WT_NB * WT_N + (size_t)2 * nt * 256 + 6 * nt) * sizeof(R); }
 
 // ------------------------------------------------------------------------
 // Rows pass with tensor-memory-accelerator (TMA) tiles: the same arithmetic
