@@ -1,0 +1,11 @@
+// C entries of the convolution kernels' plans (csrc/conv_plan.cuh) for the test.
+#include "conv_plan.cuh"
+using namespace xbg::nn;
+extern "C" {
+int rows_stages(int bn, int wc, int W, int cin) { return conv_rows_stages(bn, wc, W, cin); }
+int rows_smem(int bn, int wc, int cin, int nst) { return conv_rows_smem(bn, wc, cin, nst); }
+int rows_cols(int bn) { return conv_rows_cols(bn); }
+int wgrad_slots(int bn, int wc, int nseg) { return wgrad_rows_slots(bn, wc, nseg); }
+int wgrad_smem(int bn, int wc, int nx) { return wgrad_rows_smem(bn, wc, nx); }
+int wgrad_cols(int bn) { return wgrad_rows_cols(bn); }
+}

@@ -1,0 +1,65 @@
+"""What the box-fed convolution and weight-gradient kernels ask of an SM, over
+every channel count and width that they take: no mix of CTAs whose shared memory
+fits on an SM -- of these kernels and of the other tensor-core kernels, as launches
+on several streams put them together -- asks for more than its 512 tensor memory
+columns, so that no allocation waits."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SM, CTA_MAX, COLS = 228 * 1024, 227 * 1024, 512
+WIDTHS = (16, 32, 48, 64, 96, 128)
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("plan") / "plan.so")
+    r = subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", "-Werror", "-shared", "-fPIC",
+                        "-I", os.path.join(ROOT, "xbeach_gpu_b200", "csrc"),
+                        os.path.join(ROOT, "tests", "cxx", "conv_plan.cpp"), "-o", so], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return C.CDLL(so)
+
+
+def _rows(plan):
+    """(output channels, box channels, input channels, stages) of every layer the kernel over rows takes"""
+    for bn in WIDTHS:
+        for cin in range(16, 400, 16):
+            for wc in (64, 32, 16):
+                n = plan.rows_stages(bn, wc, 128, cin) if cin % wc == 0 else 0
+                if n:
+                    yield bn, wc, cin, n
+
+
+def _wgrad(plan):
+    for bn in WIDTHS:
+        for wc in (32, 16):
+            for nseg in range(1, 20):
+                n = plan.wgrad_slots(bn, wc, nseg)
+                if n:
+                    yield bn, wc, n
+
+
+def test_plans_fit_a_block(plan):
+    rows, wg = list(_rows(plan)), list(_wgrad(plan))
+    assert (32, 16, 16, 18) in rows and (64, 64, 64, 9) in rows and (32, 32, 13) in wg
+    for bn, wc, cin, n in rows:
+        assert 1024 + n * 256 * wc + 18 * cin * bn <= plan.rows_smem(bn, wc, cin, n) <= CTA_MAX - 1024
+    for bn, wc, n in wg:
+        assert 1024 + n * 512 * wc + 384 * bn <= plan.wgrad_smem(bn, wc, n) <= CTA_MAX - 512
+
+
+def test_no_mix_of_blocks_exceeds_tensor_memory(plan):
+    items = {(plan.rows_smem(bn, wc, cin, n) + 1024, plan.rows_cols(bn)) for bn, wc, cin, n in _rows(plan)}
+    items |= {(plan.wgrad_smem(bn, wc, n) + 1024, plan.wgrad_cols(bn)) for bn, wc, n in _wgrad(plan)}
+    # the gathered kernels and the tiled one: stages of 64 channels of 128 pixels and of the weights
+    for bn in WIDTHS + (192, 256):
+        items.add((3 * 128 * (128 + bn) + 2048, max(32, 1 << (bn - 1).bit_length())))
+    items |= {(st * 128 * (128 + bn) + 2048, bn) for bn, st in ((128, 6), (128, 3), (64, 8), (64, 4))}
+    best = [0] * (SM // 256 + 1)   # most columns in this much shared memory
+    for s in range(1, len(best)):
+        best[s] = max([best[s - 1]] + [best[s - b // 256] + c for b, c in items if b // 256 <= s])
+    assert best[-1] <= COLS

@@ -29,6 +29,7 @@
 
 #include "../../include/xbg.h"
 #include "../../include/xbg_nn.h"
+#include "conv_plan.cuh"
 
 namespace xbg {
 namespace nn {
@@ -751,24 +752,15 @@ __device__ __forceinline__ void store_cols(unsigned taddr, const float* bias, vo
 // At 512 x 1024 pixels, against k_conv_tma: 32 -> 32 channels 65 -> 32 us, 96 -> 32
 // 147 -> 66, 16 -> 32 52 -> 27; at 256 x 512, 64 -> 64 38 -> 20.  What is left is
 // the issue of the products: 55 to 90 cycles each at 16 to 64 output channels.
-constexpr int CR_MAXST = 18;      // input stages at most
 constexpr int CR_THREADS = 192;
-
-template <int BN>
-struct ConvRows {
-    // accumulator slots (three rows under way, at least one being stored) of
-    // STRIDE tensor-memory columns
-    static constexpr int STRIDE = BN <= 32 ? 32 : (BN <= 64 ? 64 : 128);
-    static constexpr int NS = BN <= 64 ? 8 : 4;
-    static constexpr int COLS = NS * STRIDE;
-};
 
 template <int BN, int WC>
 __global__ void __launch_bounds__(CR_THREADS, 1)
     k_conv_rows(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* __restrict__ Wt,
                 const float* __restrict__ bias, void* Y, int Bn, int H, int W, int cin, int ldw, int ldy, int flags,
                 int nst, int* err) {
-    constexpr int NS = ConvRows<BN>::NS, STRIDE = ConvRows<BN>::STRIDE, TCOLS = ConvRows<BN>::COLS;
+    // accumulator slots of STRIDE tensor-memory columns
+    constexpr int NS = conv_rows_slots(BN), STRIDE = conv_rows_stride(BN), TCOLS = conv_rows_cols(BN);
     constexpr int BOX = GM * WC * 2;              // bytes of a box: 128 pixels of WC channels
     constexpr int CHUNK = BN * WC * 2;            // bytes of the weights of one tap and channel group
     extern __shared__ unsigned char smem_raw[];
@@ -958,18 +950,6 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS));
 }
 
-// stages that fit beside the weights of a layer (0: k_conv_rows does not apply)
-template <int BN, int WC>
-int conv_rows_stages(int W, int cin) {
-    // the last strip of a row may be ragged; strips of which over a third lies outside the image are not worth it
-    const int strips = (W + GM - 1) / GM;
-    if (BN > 128 || W < GM || 2 * strips * GM > 3 * W) return 0;
-    const int room = 225 * 1024 - 1024 - 9 * cin * BN * 2, box = GM * WC * 2;
-    const int n = room < 0 ? 0 : room / box;
-    const int nb = 3 * (cin / WC);   // an input row's boxes are waited for together; two rows' worth, or nearly
-    return nb > 30 || n < nb + (nb + 1) / 2 ? 0 : (n > CR_MAXST ? CR_MAXST : n);
-}
-
 template <int BN, int WC>
 int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
                      int ldw, int ldy, int flags, int nst, int* err, cudaStream_t st) {
@@ -978,13 +958,13 @@ int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, vo
         int dev = 0, n = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaFuncSetAttribute(k_conv_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024) !=
+            cudaFuncSetAttribute(k_conv_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, CR_SMEM) !=
                 cudaSuccess)
             return XBG_ERR_CUDA;
         sms = n;
     }
     const long long total = (long long)Bn * ((W + GM - 1) / GM) * H;
-    const size_t smem = 1024 + (size_t)nst * GM * WC * 2 + (size_t)9 * cin * BN * 2;
+    const size_t smem = (size_t)conv_rows_smem(BN, WC, cin, nst);
     k_conv_rows<BN, WC><<<(unsigned)(total < sms ? total : sms), CR_THREADS, smem, st>>>(
         m, (const __nv_bfloat16*)Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err);
     return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA;
@@ -1189,13 +1169,13 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
         // times instead of nine)
         if (g_conv_tma) {
             int nst = 0;
-            if (cin % 64 == 0 && (nst = conv_rows_stages<BN, 64>(W, cin)) &&
+            if (cin % 64 == 0 && (nst = conv_rows_stages(BN, 64, W, cin)) &&
                 conv_map<64>(X, Bn, H, W, cin, ldx, &m, true))
                 return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
-            if (cin % 32 == 0 && (nst = conv_rows_stages<BN, 32>(W, cin)) &&
+            if (cin % 32 == 0 && (nst = conv_rows_stages(BN, 32, W, cin)) &&
                 conv_map<32>(X, Bn, H, W, cin, ldx, &m, true))
                 return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
-            if (cin % 32 != 0 && cin % 16 == 0 && (nst = conv_rows_stages<BN, 16>(W, cin)) &&
+            if (cin % 32 != 0 && cin % 16 == 0 && (nst = conv_rows_stages(BN, 16, W, cin)) &&
                 conv_map<16>(X, Bn, H, W, cin, ldx, &m, true))
                 return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
         }
@@ -1481,9 +1461,6 @@ __global__ void k_wgrad_reduce(const float* __restrict__ part, float* __restrict
 // -> 40, 128 -> 128 at 4 x 64 x 64 16 -> 12.  Runs down 64-pixel columns, which copy
 // fewer surrounding rows, took 22 us for the first of these, but sum in another order,
 // and Adam's normalised steps carry the last bits of a small gradient into the weights.
-constexpr int WR_P = 64;    // pixels of a chunk
-constexpr int WR_MX = 24;   // input slots at most
-constexpr int WR_ND = 3;    // dz slots
 
 // [B, H, W, ld] channels-last in boxes of WC channels x 64 pixels
 template <int WC>
@@ -1511,7 +1488,7 @@ __global__ void __launch_bounds__(192, 1)
     constexpr unsigned XG = WC * 2 * 8, ZG = WB * 2 * 8;   // bytes of eight pixels
     constexpr unsigned XB = WR_P * WC * 2, ZB = WR_P * WB * 2;   // bytes of a box
     constexpr unsigned XS = 4 * XB, ZS = WR_P * BN * 2;    // bytes of a slot
-    constexpr int TCOLS = BN <= 16 ? 64 : (BN <= 32 ? 128 : (BN <= 64 ? 256 : 512));
+    constexpr int TCOLS = wgrad_rows_cols(BN);
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long xfull[WR_MX], xempty[WR_MX], zfull[ND], zempty[ND], done;
     __shared__ unsigned tmem_slot;
@@ -1683,13 +1660,10 @@ __global__ void __launch_bounds__(192, 1)
 template <int BN, int WC>
 bool wgrad_rows_launch(const void* X, const void* Dz, float* work, int Bn, int H, int W, int cin, int ldx, int ldz,
                        int ldp, int bias_row, int ksplit, int* err, cudaStream_t st, int* rc) {
-    constexpr int XS = 4 * WR_P * WC * 2, MAXB = 226 * 1024;
     const int nseg = W / WR_P, chunks = Bn * H * nseg, per = (chunks + ksplit - 1) / ksplit;
-    // the resident chunks and two to four copies ahead; the rows around a run are
-    // copied too, so a run is at least as long as they are
-    const int fixed = 1024 + (WC == 16 ? XS : 0) + WR_ND * WR_P * BN * 2;
-    const int NX = std::min(std::min(2 * nseg + 5, WR_MX), (MAXB - fixed) / XS);
-    if (NX < 2 * nseg + 3 || per < 2 * nseg) return false;
+    // the rows around a run are copied too, so a run is at least as long as they are
+    const int NX = wgrad_rows_slots(BN, WC, nseg);
+    if (!NX || per < 2 * nseg) return false;
     CUtensorMap xm, zm;
     if (!strip_map<WC>(X, Bn, H, W, ldx, &xm) ||
         !strip_map<(BN % 64 == 0 ? 64 : (BN % 32 == 0 ? 32 : 16))>(Dz, Bn, H, W, ldz, &zm))
@@ -1697,12 +1671,13 @@ bool wgrad_rows_launch(const void* X, const void* Dz, float* work, int Bn, int H
     static bool attr = false;
     *rc = XBG_ERR_CUDA;
     if (!attr) {
-        if (cudaFuncSetAttribute(k_wgrad_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAXB) !=
+        if (cudaFuncSetAttribute(k_wgrad_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, WR_SMEM) !=
             cudaSuccess)
             return true;
         attr = true;
     }
-    k_wgrad_rows<BN, WC><<<dim3((unsigned)(cin / WC), (unsigned)ksplit), 192, (size_t)(fixed + NX * XS), st>>>(
+    k_wgrad_rows<BN, WC><<<dim3((unsigned)(cin / WC), (unsigned)ksplit), 192,
+                           (size_t)wgrad_rows_smem(BN, WC, NX), st>>>(
         xm, zm, work, H * nseg, nseg, chunks, per, NX, cin, ldp, bias_row, err);
     if (cudaGetLastError() == cudaSuccess) *rc = XBG_OK;
     return true;
