@@ -63,3 +63,11 @@ def test_no_mix_of_blocks_exceeds_tensor_memory(plan):
     for s in range(1, len(best)):
         best[s] = max([best[s - 1]] + [best[s - b // 256] + c for b, c in items if b // 256 <= s])
     assert best[-1] <= COLS
+
+
+def test_a_rows_boxes_have_stages(plan):
+    """All boxes of an input row are in flight together, a stage and a barrier each:
+    112 and 144 input channels (21 and 27 boxes) have more than the 18 stages."""
+    for bn, wc, cin, n in _rows(plan):
+        assert 3 * (cin // wc) <= n <= 18, (bn, wc, cin, n)
+    assert (16, 16, 80, 18) in list(_rows(plan))

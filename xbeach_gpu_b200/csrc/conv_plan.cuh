@@ -54,6 +54,7 @@ XBG_PLAN int conv_rows_stages(int bn, int wc, int W, int cin) {
     const int n = room < 0 ? 0 : room / box;
     if (n < nb + (nb + 1) / 2) return 0;
     const int nst = n > CR_MAXST ? CR_MAXST : n;
+    if (nst < nb) return 0;
     // 512 columns in a CTA that needs less than half of the SM's shared memory (16
     // input channels, 48 to 128 output channels): left to the other kernels
     if (2 * conv_rows_cols(bn) > SM_TCOLS && 2 * (conv_rows_bytes(bn, wc, cin, nst) + 1024) <= SM_SMEM) return 0;
