@@ -30,6 +30,7 @@
 #include "../../include/xbg.h"
 #include "../../include/xbg_nn.h"
 #include "conv_plan.cuh"
+#include "copy_ring.cuh"
 
 namespace xbg {
 namespace nn {
@@ -686,6 +687,19 @@ __device__ __forceinline__ bool role_wait(unsigned a, unsigned parity, int* bad)
     *(volatile int*)bad = 1;
     return false;
 }
+// Leaving early: the last copy into each of a ring's slots lands first, a lane per
+// slot (bounded).  n and `some` as in ring_last, the same in every lane.
+__device__ __forceinline__ void drain_copies(unsigned long long* full, int slots, int n, unsigned some, int lane) {
+    if (lane < slots) {
+        const int q = ring_last(n, some, slots, lane);
+        if (q >= 0) mbar_wait(smem_u32(&full[lane]), ring_parity(q, slots));
+    }
+    __syncwarp();
+}
+// the value of the lane that issues (each lane counts its own way through the loop)
+__device__ __forceinline__ int of_leader(int v, unsigned leader) {
+    return __shfl_sync(0xffffffffu, v, __ffs((int)__ballot_sync(0xffffffffu, leader != 0)) - 1);
+}
 // CW accumulator columns of this warp's 32 tensor-memory lanes (one pixel per
 // lane) in registers
 template <int CW>
@@ -747,8 +761,9 @@ __device__ __forceinline__ void store_cols(unsigned taddr, const float* bias, vo
 //    products.
 // Warp 0 issues the copies, warp 1 the products, warps 2..5 store the rows; all
 // meet on mbarriers (full / empty per stage and per accumulator slot).  Every
-// wait is bounded: a role that gives up sets a flag that ends the others' waits,
-// and the CTA leaves after its copies and products in flight (bounded again).
+// wait is bounded: a role that gives up sets a flag that ends the others' waits;
+// once every role has ended, the flag is final, and with it set the CTA leaves
+// after all its copies and products in flight (bounded again).
 // At 512 x 1024 pixels, against k_conv_tma: 32 -> 32 channels 65 -> 32 us, 96 -> 32
 // 147 -> 66, 16 -> 32 52 -> 27; at 256 x 512, 64 -> 64 38 -> 20.  What is left is
 // the issue of the products: 55 to 90 cycles each at 16 to 64 output channels.
@@ -817,11 +832,19 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
             l += n;
         }
     };
+    int sent = 0;        // copies issued, in whole rows; of the row a wait ended, the lanes that issued
+    unsigned some = 0;
+    // one lane's commit covers what it issued before
+    auto commit = [&](const void* bar) {
+        if (leader) asm volatile(
+            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar))
+            : "memory");
+    };
     if (warp == 0) {
         // ---- copies: lane c takes box c of an input row (dx, channel group)
         const int cx = lane / ncg - 1, cch = lane % ncg * WC;
-        int s = 0, mine = -1;   // the row's first stage; the stage this lane used last
-        unsigned ph = 0, minep = 0;
+        int s = 0;   // the row's first stage
+        unsigned ph = 0;
         segments([&](int b, int x0, int y0, int n, int) {
             for (int r = y0 - 1; r <= y0 + n; r++) {
                 bool ok = true;
@@ -839,29 +862,22 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
                             "[%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(base + (unsigned)t * BOX),
                             "l"((unsigned long long)&xmap), "r"(cch), "r"(x0 + cx), "r"(r), "r"(b), "r"(fb)
                             : "memory");
-                        mine = t;
-                        minep = tp;
                     }
                 }
-                if (!__all_sync(0xffffffffu, ok)) return false;
+                if (!__all_sync(0xffffffffu, ok)) {
+                    some = __ballot_sync(0xffffffffu, ok && lane < nb);
+                    return false;
+                }
+                sent += nb;
                 s += nb;
                 if (s >= nst) { s -= nst; ph ^= 1u; }
             }
             return true;
         });
-        // leaving early: every stage's copy in flight lands first.  A lane's last
-        // box lands after its earlier ones have been waited for by the products
-        // or are older than it in the same queue; the bounded wait covers both.
-        if (*(volatile int*)&bad && mine >= 0) mbar_wait(smem_u32(&full[mine]), minep);
     } else if (warp == 1) {   // ---- products: the warp runs in step, one lane issues
         const uint32_t idesc = idesc_bf16(GM, BN);
         const uint64_t da0 = swk_desc<WC>(base), db0 = swk_desc<WC>(wbase);
         const uint64_t tstep = (uint64_t)(3 * ncg * CHUNK >> 4);   // from a tap row's weights to the next one's
-        auto commit = [&](const void* bar) {
-            if (leader) asm volatile(
-                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar))
-                : "memory");
-        };
         auto mma = [&](unsigned d, uint64_t da, uint64_t db, unsigned acc) {
             if (leader) asm volatile(
                 "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -913,10 +929,6 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
             }
             return true;
         });
-        if (*(volatile int*)&bad) {   // products in flight end before tensor memory goes
-            commit(&drain);
-            mbar_wait(smem_u32(&drain), 0);
-        }
     } else {   // ---- rows out: warp w reads tensor memory lanes 32 (w % 4) ..
         const int q = warp & 3;
         segments([&](int b, int x0, int y0, int n, int o0) {
@@ -943,8 +955,15 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
             return true;
         });
     }
-    __syncthreads();
-    if (tid == 0 && bad) atomicExch(err, XBG_ERR_TIMEOUT);
+    __syncthreads();   // every role has ended: `bad` is final
+    if (bad) {         // a wait ran out: copies and products in flight end before shared and tensor memory go
+        if (warp == 0) drain_copies(full, nst, sent, some, lane);
+        if (warp == 1) {
+            commit(&drain);
+            mbar_wait(smem_u32(&drain), 0);
+        }
+        if (tid == 0) atomicExch(err, XBG_ERR_TIMEOUT);
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS));
@@ -1018,11 +1037,12 @@ __global__ void __launch_bounds__(192, 1)
     unsigned leader;   // one lane of each warp
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
     auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
+    int sent = 0;   // chunks whose copies were issued
     if (warp == 0) {   // ---- copies
         const unsigned bytes = (unsigned)(R * Wt) * GK * 2 + B_BYTES;
-        int s = 0, c0 = 0, dx = -1, dy = -1, kc = 0;
+        int s = 0, c0 = 0, dx = -1, dy = -1;
         unsigned ph = 0;
-        for (; kc < nk; kc++) {
+        for (int kc = 0; kc < nk; kc++) {
             if (!wait(smem_u32(&empty[s]), ph ^ 1u)) break;
             if (leader) {
                 const unsigned fb = smem_u32(&full[s]), sa = base + (unsigned)s * STAGE;
@@ -1039,6 +1059,7 @@ __global__ void __launch_bounds__(192, 1)
                     "l"((unsigned long long)&wmap), "r"(kc * GK), "r"(n0), "r"(fb)
                     : "memory");
             }
+            sent++;
             if (++s == ST) { s = 0; ph ^= 1u; }
             c0 += GK;
             if (c0 == cin) {
@@ -1046,8 +1067,6 @@ __global__ void __launch_bounds__(192, 1)
                 if (++dx == 2) { dx = -1; dy++; }
             }
         }
-        if (*(volatile int*)&bad)   // leaving early: the copies in flight land first (bounded)
-            for (int c = max(kc - ST, 0); c < kc; c++) mbar_wait(smem_u32(&full[c % ST]), (c / ST) & 1);
     } else if (warp == 1) {   // ---- products
         const uint32_t idesc = idesc_bf16(GM, BN);
         const uint64_t a0 = sw128_desc(base), b0 = sw128_desc(base + A_BYTES);
@@ -1075,7 +1094,6 @@ __global__ void __launch_bounds__(192, 1)
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
                              smem_u32(&done))
                          : "memory");
-        if (*(volatile int*)&bad) mbar_wait(smem_u32(&done), 0);
     } else {   // ---- the tile out
         const int q = warp & 3;
         if (__all_sync(0xffffffffu, wait(smem_u32(&done), 0)) && !*(volatile int*)&bad) {
@@ -1091,8 +1109,15 @@ __global__ void __launch_bounds__(192, 1)
             }
         }
     }
-    __syncthreads();
-    if (tid == 0 && bad) atomicExch(err, XBG_ERR_TIMEOUT);
+    __syncthreads();   // every role has ended: `bad` is final
+    if (bad) {         // as in k_conv_rows
+        if (warp == 0) {
+            __syncwarp();
+            drain_copies(full, ST, of_leader(sent, leader), 0, lane);
+        }
+        if (warp == 1) mbar_wait(smem_u32(&done), 0);
+        if (tid == 0) atomicExch(err, XBG_ERR_TIMEOUT);
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN));
@@ -1526,6 +1551,7 @@ __global__ void __launch_bounds__(192, 1)
     unsigned leader;   // one lane of each warp
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
     auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
+    int nxl = 0, nzl = 0;   // input and dz chunks whose copies were issued
     if (warp == 0) {   // ---- copies: per image of the run, input chunks i0 - nseg .. i1 - 1 + nseg, dz chunks i0 .. i1 - 1
         auto box = [&](unsigned dst, const CUtensorMap* m, int c, int x, int y, int b, unsigned bar) {
             asm volatile(
@@ -1534,7 +1560,7 @@ __global__ void __launch_bounds__(192, 1)
                 "l"((unsigned long long)m), "r"(c), "r"(x), "r"(y), "r"(b), "r"(bar)
                 : "memory");
         };
-        int xs = 0, zs = 0, nxl = 0, nzl = 0;
+        int xs = 0, zs = 0;
         unsigned xp = 0, zp = 0;
         bool go = true;
         for (int u = u0; u < u1 && go;) {
@@ -1564,10 +1590,6 @@ __global__ void __launch_bounds__(192, 1)
                 if (++zsg == nseg) { zsg = 0; zy++; }
             }
             u += n;
-        }
-        if (*(volatile int*)&bad) {   // leaving early: the copies in flight land first (bounded)
-            for (int k = max(nxl - NX, 0); k < nxl; k++) mbar_wait(smem_u32(&xfull[k % NX]), (k / NX) & 1);
-            for (int k = max(nzl - ND, 0); k < nzl; k++) mbar_wait(smem_u32(&zfull[k % ND]), (k / ND) & 1);
         }
     } else if (warp == 1) {   // ---- products
         const uint32_t idesc = idesc_bf16(GM, BN) | (1u << 15) | (1u << 16);   // A and B MN-major
@@ -1623,7 +1645,6 @@ __global__ void __launch_bounds__(192, 1)
             u += n;
         }
         commit(&done);   // every product issued so far
-        if (*(volatile int*)&bad) mbar_wait(smem_u32(&done), 0);
     } else {   // ---- accumulator row m of y offset dy: x offset m / WC, channel m % WC
         const int q = warp & 3;
         if (__all_sync(0xffffffffu, wait(smem_u32(&done), 0)) && !*(volatile int*)&bad) {
@@ -1648,8 +1669,16 @@ __global__ void __launch_bounds__(192, 1)
                 }
         }
     }
-    __syncthreads();
-    if (tid == 0 && bad) atomicExch(err, XBG_ERR_TIMEOUT);
+    __syncthreads();   // every role has ended: `bad` is final
+    if (bad) {         // as in k_conv_rows
+        if (warp == 0) {
+            __syncwarp();
+            drain_copies(xfull, NX, of_leader(nxl, leader), 0, lane);
+            drain_copies(zfull, ND, of_leader(nzl, leader), 0, lane);
+        }
+        if (warp == 1) mbar_wait(smem_u32(&done), 0);
+        if (tid == 0) atomicExch(err, XBG_ERR_TIMEOUT);
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 1)
