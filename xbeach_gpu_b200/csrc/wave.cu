@@ -1382,25 +1382,32 @@ __device__ __forceinline__ void b_wave_tma(const Dev<R>& S, const Konst<R>& K, c
     block_min_store<R>(dtw, S.part_wave + bix + biy * ((K.nx + 31) / 32));
 }
 // Threads and cells.  FP32 with the roller: two cells and both fields per thread
-// (128 threads, 111 registers, four blocks per SM by shared memory at 18 bins);
+// (128 threads, 109 registers, four blocks per SM by shared memory at 18 bins);
 // four cells of one field on as many threads take 306 against 285 us at
 // 2048 x 1024, four cells of both on 64 threads leave too few warps (332 us).
 // FP64: two cells (16-byte loads at most) of one field on 256 threads (66
 // against 74 us at 512 x 256 for both fields on 128).  Without the roller a
 // thread has four (FP64: two) cells.
+// Blocks per SM: FP64 without the roller has 128 threads, and with two blocks
+// (190 registers) an SM had eight warps; with three (155 registers) the pass takes
+// 101 against 128 us at 1024 x 512 x 4 bins and 179 against 223 at 18 (one cell per
+// thread: 107 and 231), ten ragged domains of 8 bins 739 against 842 (860).  Four
+// (128 registers) are faster still up to 18 bins (93 and 169 us) and slower at 24
+// and more (224 against 212, 344 against 320).
 template <class R, bool ROLLER> constexpr bool wave_split = ROLLER && sizeof(R) == 8;
 template <class R, bool ROLLER> constexpr int wave_v = sizeof(R) == 8 || ROLLER ? 2 : 4;
 template <class R, bool ROLLER>
 constexpr int wave_threads = (wave_split<R, ROLLER> ? 512 : 256) / wave_v<R, ROLLER>;
+template <class R, bool ROLLER> constexpr int wave_min_blocks = sizeof(R) == 4 ? 4 : (ROLLER ? 2 : 3);
 template <class R, bool ROLLER>
-__global__ void __launch_bounds__(wave_threads<R, ROLLER>, sizeof(R) == 4 ? 4 : 2)
+__global__ void __launch_bounds__(wave_threads<R, ROLLER>, wave_min_blocks<R, ROLLER>)
     k_wave_tma(Dev<R> S, Konst<R> K, const __grid_constant__ WaveMaps M) {
     b_wave_tma<R, ROLLER, wave_v<R, ROLLER>, wave_split<R, ROLLER>>(S, K, M, blockIdx.x, blockIdx.y);
 }
 // every scenario of a batch: its tensor maps from a device array (written
 // by the host before the first launch), one per scenario
 template <class R, bool ROLLER>
-__global__ void __launch_bounds__(wave_threads<R, ROLLER>, sizeof(R) == 4 ? 4 : 2)
+__global__ void __launch_bounds__(wave_threads<R, ROLLER>, wave_min_blocks<R, ROLLER>)
     kb_wave_tma(BatchTab<R> T, const WaveMaps* __restrict__ maps, const int2* items, int n) {
     batch_items<R>(T, items, n, [&](const Dev<R>& S, const Konst<R>& K, const BatchAux& A, int bx, int by) {
         b_wave_tma<R, ROLLER, wave_v<R, ROLLER>, wave_split<R, ROLLER>>(S, K, maps[A.scen], bx, by);
