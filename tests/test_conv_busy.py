@@ -10,9 +10,22 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("cin,N", [(16, 48), (16, 64), (16, 96), (16, 128), (48, 48), (32, 96), (32, 128), (64, 128)])
 def test_conv_all_sms(cin, N):
+    _conv(4, 256, 256, cin, N)
+
+
+# runs of rows that end with their strip and runs that cross into the next one (the
+# last of a strip shorter, one row longer than the rows divide, more strips than SMs),
+# ragged strips, and 16-channel boxes at the smallest size that takes them and below
+@pytest.mark.parametrize("B,H,W,cin,N", [(1, 256, 256, 16, 32), (1, 224, 224, 16, 32), (1, 400, 400, 16, 16),
+                                         (2, 250, 300, 48, 48), (1, 304, 300, 96, 32), (1, 160, 176, 32, 32),
+                                         (1, 208, 256, 64, 128), (4, 240, 254, 32, 64), (150, 3, 128, 64, 64)])
+def test_conv_runs(B, H, W, cin, N):
+    _conv(B, H, W, cin, N)
+
+
+def _conv(B, H, W, cin, N):
     import torch
     from xbeach_gpu_b200 import surrogate as sg
-    B, H, W = 4, 256, 256
     g = torch.Generator(device="cuda").manual_seed(cin + N)
     L = sg.lib()
     P, Kp = B * H * W, (9 * cin + 63) // 64 * 64

@@ -71,3 +71,28 @@ def test_a_rows_boxes_have_stages(plan):
     for bn, wc, cin, n in _rows(plan):
         assert 3 * (cin // wc) <= n <= 18, (bn, wc, cin, n)
     assert (16, 16, 80, 18) in list(_rows(plan))
+
+
+@pytest.mark.parametrize("extra", [0, 1])
+def test_runs_cover_every_row_once(plan, extra):
+    """The runs of the blocks are the rows of all strips in order, each once, none
+    empty, on at most one block per SM; and no block reads more input rows (two more
+    than it writes, per strip that it touches) than runs on end would give it."""
+    for sms in (1, 7, 132, 148):
+        for S in (1, 2, 3, 4, 7, 8, 12, 40, 147, 148, 149, 300):
+            for H in (1, 2, 3, 5, 16, 37, 100, 127, 160, 208, 256, 304, 512, 1000):
+                buf = (C.c_int * (2 * sms))()
+                n = plan.rows_run(S, H, sms, extra, None)
+                assert 1 <= n <= sms
+                plan.rows_run(S, H, sms, extra, buf)
+                runs = [(buf[2 * k], buf[2 * k + 1]) for k in range(n)]
+                assert runs[0][0] == 0 and runs[-1][1] == S * H
+                assert all(a < b for a, b in runs) and all(p[1] == q[0] for p, q in zip(runs, runs[1:]))
+
+                def most(rs):
+                    return max(b - a + 2 * ((b - 1) // H - a // H + 1) for a, b in rs)
+                per = -(-S * H // sms)
+                assert most(runs) <= most([(k, min(S * H, k + per)) for k in range(0, S * H, per)])
+                assert max(b - a for a, b in runs) <= per + extra
+    buf = (C.c_int * 296)()
+    assert plan.rows_run(2, 160, 148, 0, buf) == 108 and (buf[2], buf[3]) == (3, 6) and (buf[108], buf[109]) == (160, 163)

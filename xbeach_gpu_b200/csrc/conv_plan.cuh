@@ -60,6 +60,40 @@ XBG_PLAN int conv_rows_stages(int bn, int wc, int W, int cin) {
     if (2 * conv_rows_cols(bn) > SM_TCOLS && 2 * (conv_rows_bytes(bn, wc, cin, nst) + 1024) <= SM_SMEM) return 0;
     return nst;
 }
+// 16-channel boxes (32 bytes a pixel) pay from three rows a CTA on, with 16 output
+// channels from four: below, k_conv_tma's and k_conv_tc's blocks, two and more to an
+// SM, end first.  16 -> 32 channels at 128 x 128 pixels 5.5 us there, 6.5 here, at
+// 208 x 256 7.6, 8.4, at 256 x 256 10.5, 9.0; 48 -> 16 at 256 x 256 13.9, 15.3, at
+// 240 x 344 19.2, 16.7.  Wider boxes are the faster at every size.
+XBG_PLAN bool conv_rows_pays(int bn, int wc, long long pixels, int sms) {
+    return wc > 16 || pixels >= (bn == 16 ? 4LL : 3LL) * PLAN_GM * sms;
+}
+// A CTA's run: `per` consecutive output rows of the S = images x strips strips of H
+// rows, `cps` CTAs to a strip, or runs on end across strips (cps 0).  A run of n
+// rows in one strip reads n + 2 input rows, one that crosses into the next strip
+// n + 4, so runs keep to a strip where that makes them no longer, or one row longer
+// in a layer whose time is its copies (extra).  48 -> 48 channels at 160 x 176 pixels
+// 19.9 us with runs across strips, 14.7 without; 32 -> 32 at 2 x 256 x 256 13.0, 11.1
+// (7 rows either way); 96 -> 32 at 240 x 1016 36.7, 34.4 (13 rows, 14); where products
+// bound the layer 14 rows for 13 lose: 64 -> 128 there 36.7, 38.2.
+struct RowsRun { int per, cps; };
+XBG_PLAN RowsRun conv_rows_run(int S, int H, int sms, bool extra) {
+    const int per = (int)(((long long)S * H + sms - 1) / sms);
+    if (H % per != 0 && S <= sms) {
+        const int c = sms / S, p = (H + c - 1) / c;
+        if (p <= per + (extra ? 1 : 0)) return RowsRun{p, (H + p - 1) / p};
+    }
+    return RowsRun{per, 0};
+}
+XBG_PLAN int conv_rows_ctas(RowsRun r, int S, int H) {
+    return r.cps ? S * r.cps : (int)(((long long)S * H + r.per - 1) / r.per);
+}
+// first and last (exclusive) row of a CTA's run
+XBG_PLAN int conv_rows_lo(RowsRun r, int H, int cta) { return r.cps ? cta / r.cps * H + cta % r.cps * r.per : cta * r.per; }
+XBG_PLAN int conv_rows_hi(RowsRun r, int S, int H, int cta) {
+    const int hi = conv_rows_lo(r, H, cta) + r.per, end = r.cps ? (cta / r.cps + 1) * H : S * H;
+    return hi < end ? hi : end;
+}
 
 // ---- k_wgrad_rows
 XBG_PLAN int wgrad_rows_cols(int bn) { return bn <= 16 ? 64 : (bn <= 32 ? 128 : (bn <= 64 ? 256 : 512)); }

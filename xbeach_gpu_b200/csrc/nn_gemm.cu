@@ -764,8 +764,8 @@ __device__ __forceinline__ void store_cols(unsigned taddr, const float* bias, vo
 // wait is bounded: a role that gives up sets a flag that ends the others' waits;
 // once every role has ended, the flag is final, and with it set the CTA leaves
 // after all its copies and products in flight (bounded again).
-// At 512 x 1024 pixels, against k_conv_tma: 32 -> 32 channels 65 -> 32 us, 96 -> 32
-// 147 -> 66, 16 -> 32 52 -> 27; at 256 x 512, 64 -> 64 38 -> 20.  What is left is
+// At 512 x 1024 pixels, against k_conv_tma: 32 -> 32 channels 64 -> 30 us, 96 -> 32
+// 146 -> 64, 16 -> 32 51 -> 25; at 256 x 512, 64 -> 64 38 -> 18.  What is left is
 // the issue of the products: 55 to 90 cycles each at 16 to 64 output channels.
 constexpr int CR_THREADS = 192;
 
@@ -773,7 +773,7 @@ template <int BN, int WC>
 __global__ void __launch_bounds__(CR_THREADS, 1)
     k_conv_rows(const __grid_constant__ CUtensorMap xmap, const __nv_bfloat16* __restrict__ Wt,
                 const float* __restrict__ bias, void* Y, int Bn, int H, int W, int cin, int ldw, int ldy, int flags,
-                int nst, int* err) {
+                int nst, RowsRun run, int* err) {
     // accumulator slots of STRIDE tensor-memory columns
     constexpr int NS = conv_rows_slots(BN), STRIDE = conv_rows_stride(BN), TCOLS = conv_rows_cols(BN);
     constexpr int BOX = GM * WC * 2;              // bytes of a box: 128 pixels of WC channels
@@ -784,10 +784,8 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
     __shared__ int bad;
     __shared__ float sbias[BN];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int strips = (W + GM - 1) / GM, total = Bn * strips * H, ncg = cin / WC, nb = 3 * ncg;   // boxes of an input row
-    const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int lo = (int)blockIdx.x * per, hi = min(total, lo + per);
-    if (lo >= hi) return;   // the whole CTA
+    const int strips = (W + GM - 1) / GM, ncg = cin / WC, nb = 3 * ncg;   // boxes of an input row
+    const int lo = conv_rows_lo(run, H, (int)blockIdx.x), hi = conv_rows_hi(run, Bn * strips, H, (int)blockIdx.x);
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const unsigned wbase = base + (unsigned)nst * BOX;   // the weights, [tap][channel group][BN][WC]
 
@@ -969,23 +967,33 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS));
 }
 
-template <int BN, int WC>
-int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
-                     int ldw, int ldy, int flags, int nst, int* err, cudaStream_t st) {
-    static int sms = 0;   // attribute and SM count: the same for every caller
+// SMs of the device, 0 on an error
+inline int sm_count() {
+    static int sms = 0;
     if (!sms) {
         int dev = 0, n = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaFuncSetAttribute(k_conv_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, CR_SMEM) !=
-                cudaSuccess)
-            return XBG_ERR_CUDA;
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return 0;
         sms = n;
     }
-    const long long total = (long long)Bn * ((W + GM - 1) / GM) * H;
-    const size_t smem = (size_t)conv_rows_smem(BN, WC, cin, nst);
-    k_conv_rows<BN, WC><<<(unsigned)(total < sms ? total : sms), CR_THREADS, smem, st>>>(
-        m, (const __nv_bfloat16*)Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err);
+    return sms;
+}
+
+template <int BN, int WC>
+int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
+                     int ldw, int ldy, int flags, int nst, int sms, int* err, cudaStream_t st) {
+    static bool attr = false;
+    if (!attr) {
+        if (cudaFuncSetAttribute(k_conv_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, CR_SMEM) !=
+            cudaSuccess)
+            return XBG_ERR_CUDA;
+        attr = true;
+    }
+    const int S = Bn * ((W + GM - 1) / GM);
+    const RowsRun run = conv_rows_run(S, H, sms, BN <= 32 || BN <= cin);
+    k_conv_rows<BN, WC><<<(unsigned)conv_rows_ctas(run, S, H), CR_THREADS, (size_t)conv_rows_smem(BN, WC, cin, nst), st>>>(
+        m, (const __nv_bfloat16*)Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, run, err);
     return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA;
 }
 
@@ -1194,15 +1202,18 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
         // times instead of nine)
         if (g_conv_tma) {
             int nst = 0;
+            const int sms = sm_count();
+            if (!sms) return XBG_ERR_CUDA;
             if (cin % 64 == 0 && (nst = conv_rows_stages(BN, 64, W, cin)) &&
                 conv_map<64>(X, Bn, H, W, cin, ldx, &m, true))
-                return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
+                return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, sms, err, st);
             if (cin % 32 == 0 && (nst = conv_rows_stages(BN, 32, W, cin)) &&
                 conv_map<32>(X, Bn, H, W, cin, ldx, &m, true))
-                return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
-            if (cin % 32 != 0 && cin % 16 == 0 && (nst = conv_rows_stages(BN, 16, W, cin)) &&
+                return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, sms, err, st);
+            if (cin % 32 != 0 && cin % 16 == 0 && conv_rows_pays(BN, 16, M, sms) &&
+                (nst = conv_rows_stages(BN, 16, W, cin)) &&
                 conv_map<16>(X, Bn, H, W, cin, ldx, &m, true))
-                return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, err, st);
+                return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, sms, err, st);
         }
     }
     // tile by tile in 64-channel chunks where the tiles lie inside the image for two thirds
