@@ -115,6 +115,15 @@ XBG_PLAN int wgrad_rows_slots(int bn, int wc, int nseg) {
     if (2 * wgrad_rows_cols(bn) > SM_TCOLS && 2 * (wgrad_rows_bytes(bn, wc, nx) + 1024) <= SM_SMEM) return 0;
     return nx;
 }
+// Where it pays: 32-channel boxes; 16-channel boxes for 16 input channels, and for
+// more (a block each, with its own copy of the gradient's chunks) where the rows
+// around a run are short: 48 -> 16 channels at 4 x 96 x 128 pixels 18.4 us by
+// k_wgrad_tc, 14.7 here, but at 1 x 256 x 256 21.5 and 31.2, 48 -> 48 there 27.8 and
+// 34.0.  Slices of under eight chunks are images of a few rows (128 -> 128 at 3 x 128
+// pixels 12.1 there, 13.5 here).
+XBG_PLAN bool wgrad_rows_pays(int cin, int nseg, int chunks_per_slice) {
+    return (cin % 32 == 0 || cin == 16 || nseg <= 2) && chunks_per_slice >= 8;
+}
 
 }  // namespace nn
 }  // namespace xbg

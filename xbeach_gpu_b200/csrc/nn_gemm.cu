@@ -1474,7 +1474,8 @@ __global__ void k_wgrad_reduce(const float* __restrict__ part, float* __restrict
 }
 
 // ------------------------------------------------------------------------
-// The weight gradient with box copies (W a multiple of 64, cin of 16, BN <= 128).
+// The weight gradient with box copies (W a multiple of 64, cin of 16, BN <= 128;
+// wgrad_rows_pays).
 // k_wgrad_tc gathers every 64-pixel chunk of its 128 k columns once per tap,
 // thread by thread, and its threads meet twice per chunk: about a microsecond
 // per chunk whatever it holds.  Here
@@ -1703,7 +1704,7 @@ bool wgrad_rows_launch(const void* X, const void* Dz, float* work, int Bn, int H
     const int nseg = W / WR_P, chunks = Bn * H * nseg, per = (chunks + ksplit - 1) / ksplit;
     // the rows around a run are copied too, so a run is at least as long as they are
     const int NX = wgrad_rows_slots(BN, WC, nseg);
-    if (!NX || per < 2 * nseg) return false;
+    if (!NX || per < 2 * nseg || !wgrad_rows_pays(cin, nseg, per)) return false;
     CUtensorMap xm, zm;
     if (!strip_map<WC>(X, Bn, H, W, ldx, &xm) ||
         !strip_map<(BN % 64 == 0 ? 64 : (BN % 32 == 0 ? 32 : 16))>(Dz, Bn, H, W, ldz, &zm))
