@@ -15,10 +15,12 @@ def test_conv_all_sms(cin, N):
 
 # runs of rows that end with their strip and runs that cross into the next one (the
 # last of a strip shorter, one row longer than the rows divide, more strips than SMs),
-# ragged strips, and 16-channel boxes at the smallest size that takes them and below
+# ragged strips, 16-channel boxes at the smallest size that takes them and below, and
+# tiles either side of one block per SM in slices of 64 and of 128 channels
 @pytest.mark.parametrize("B,H,W,cin,N", [(1, 256, 256, 16, 32), (1, 224, 224, 16, 32), (1, 400, 400, 16, 16),
                                          (2, 250, 300, 48, 48), (1, 304, 300, 96, 32), (1, 160, 176, 32, 32),
-                                         (1, 208, 256, 64, 128), (4, 240, 254, 32, 64), (150, 3, 128, 64, 64)])
+                                         (1, 208, 256, 64, 128), (4, 240, 254, 32, 64), (150, 3, 128, 64, 64),
+                                         (1, 74, 128, 128, 128), (1, 75, 128, 128, 128), (1, 149, 128, 128, 128)])
 def test_conv_runs(B, H, W, cin, N):
     _conv(B, H, W, cin, N)
 

@@ -31,6 +31,7 @@
 #include "../../include/xbg_nn.h"
 #include "conv_plan.cuh"
 #include "copy_ring.cuh"
+#include "per_device.cuh"
 
 namespace xbg {
 namespace nn {
@@ -40,6 +41,27 @@ constexpr int GK = 64;           // K chunk: 64 bf16 = one 128-B swizzle row
 constexpr int GSTAGES = 3;
 constexpr unsigned WAIT_LIMIT = 1u << 22;   // try_wait polls before giving up
 constexpr unsigned CHECK_WAIT_LIMIT = 4096; // polls of the time-out check (XBG_NN_CHECK_TIMEOUT)
+
+inline int current_device() {
+    int dev = -1;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+// a kernel's dynamic shared memory limit on the current device; false on an error
+template <class K>
+bool smem_limit(PerDevice& d, K kernel, int bytes) {
+    return d.get(current_device(), [&] {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    }) != 0;
+}
+// SMs of the current device, 0 on an error
+inline int sm_count() {
+    static PerDevice sms;
+    const int dev = current_device();
+    return sms.get(dev, [&] {
+        int n = 0;
+        return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 0;
+    });
+}
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -233,12 +255,8 @@ int gemm_launch(const void* A, const void* B, const float* bias, void* C, int M,
                 int ldc, int flags, int ksplit, int* err, cudaStream_t st) {
     constexpr int STAGE = GM * GK * 2 + BN * GK * 2;
     const size_t smem = (size_t)GSTAGES * STAGE + 1024;
-    static bool attr = false;   // per process; the attribute is per function
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_gemm_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return XBG_ERR_CUDA;
-        attr = true;
-    }
+    static PerDevice limit;
+    if (!smem_limit(limit, k_gemm_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
     dim3 grid((M + GM - 1) / GM, ksplit);
     k_gemm_tc<BN><<<grid, 256, smem, st>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)B, bias, C, M, N, K, lda,
                                            ldb, ldc, flags, err);
@@ -662,13 +680,8 @@ int conv_tma_launch(const CUtensorMap& m, const void* Wt, const float* bias, voi
                     int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
     constexpr int STAGE = GM * GK * 2 + BN * GK * 2;
     const size_t smem = (size_t)CSTAGES * STAGE + 1024;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_conv_tma<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess)
-            return XBG_ERR_CUDA;
-        attr = true;
-    }
+    static PerDevice limit;
+    if (!smem_limit(limit, k_conv_tma<BN, WC>, (int)smem)) return XBG_ERR_CUDA;
     const long long M = (long long)Bn * H * W;
     k_conv_tma<BN, WC><<<(unsigned)((M + GM - 1) / GM), 256, smem, st>>>(m, (const __nv_bfloat16*)Wt, bias, Y, Bn,
                                                                           H, W, cin, N, Kp, ldw, ldy, flags, err);
@@ -967,29 +980,11 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS));
 }
 
-// SMs of the device, 0 on an error
-inline int sm_count() {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return 0;
-        sms = n;
-    }
-    return sms;
-}
-
 template <int BN, int WC>
 int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
                      int ldw, int ldy, int flags, int nst, int sms, int* err, cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_conv_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, CR_SMEM) !=
-            cudaSuccess)
-            return XBG_ERR_CUDA;
-        attr = true;
-    }
+    static PerDevice limit;
+    if (!smem_limit(limit, k_conv_rows<BN, WC>, CR_SMEM)) return XBG_ERR_CUDA;
     const int S = Bn * ((W + GM - 1) / GM);
     const RowsRun run = conv_rows_run(S, H, sms, BN <= 32 || BN <= cin);
     k_conv_rows<BN, WC><<<(unsigned)conv_rows_ctas(run, S, H), CR_THREADS, (size_t)conv_rows_smem(BN, WC, cin, nst), st>>>(
@@ -1151,13 +1146,8 @@ template <int BN, int ST>
 int conv_ws_launch(const CUtensorMap& xm, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
                    int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
     constexpr size_t smem = (size_t)ST * (GM + BN) * GK * 2 + 1024;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_conv_ws<BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess)
-            return XBG_ERR_CUDA;
-        attr = true;
-    }
+    static PerDevice limit;
+    if (!smem_limit(limit, k_conv_ws<BN, ST>, (int)smem)) return XBG_ERR_CUDA;
     CUtensorMap wm;
     if (!weight_map(Wt, N, Kp, ldw, BN, &wm)) return XBG_ERR_CUDA;
     const dim3 grid((unsigned)conv_ws_tiles(Bn, H, W), (unsigned)(N / BN));
@@ -1165,14 +1155,17 @@ int conv_ws_launch(const CUtensorMap& xm, const void* Wt, const float* bias, voi
     return cudaGetLastError() == cudaSuccess ? XBG_OK : XBG_ERR_CUDA;
 }
 
-// BN of a CTA and its stages.  128 channels where the tiles then still fill most
-// SMs (the input is read once per slice), else slices of 64; one CTA per SM with
-// deep stages where the grid has no second wave, two with half of them elsewhere.
+// BN of a CTA and its stages.  Slices of 64 channels while each has an SM of its own
+// (128 -> 128 channels, 72 tiles: 7.9 us, in slices of 128 9.1), from there slices of
+// 128, which read the input once (80 tiles 9.2, in slices of 64 9.6).  One CTA per SM
+// with deep stages while the grid has no second wave (148 tiles 9.8 us, with two CTAs'
+// stages 10.1; slices of 64 the same either way), else two with half of them (150
+// tiles 12.8, with deep stages 16.4).
 inline int conv_ws(const CUtensorMap& xm, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
-                   int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
+                   int N, int Kp, int ldw, int ldy, int flags, int sms, int* err, cudaStream_t st) {
     const long long tiles = conv_ws_tiles(Bn, H, W);
-    const bool wide = N % 128 == 0 && tiles * (N / 128) >= 100;
-    const bool deep = tiles * (N / (wide ? 128 : 64)) <= 148;
+    const bool wide = N % 128 == 0 && tiles * (N / 64) > sms;
+    const bool deep = tiles * (N / (wide ? 128 : 64)) <= sms;
 #define XBG_CONV_WS(BN, ST) \
     conv_ws_launch<BN, ST>(xm, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st)
     if (wide) return deep ? XBG_CONV_WS(128, 6) : XBG_CONV_WS(128, 3);
@@ -1189,21 +1182,17 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
                 int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
     constexpr int STAGE = GM * GK * 2 + BN * GK * 2;
     const size_t smem = (size_t)CSTAGES * STAGE + 1024;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_conv_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return XBG_ERR_CUDA;
-        attr = true;
-    }
+    static PerDevice limit;
+    if (!smem_limit(limit, k_conv_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
     const long long M = (long long)Bn * H * W;
     CUtensorMap m;
+    const int sms = sm_count();
+    if (!sms) return XBG_ERR_CUDA;
     if constexpr (BN <= 128) {
         // over rows where the weights fit beside the stages (the input is read three
         // times instead of nine)
         if (g_conv_tma) {
             int nst = 0;
-            const int sms = sm_count();
-            if (!sms) return XBG_ERR_CUDA;
             if (cin % 64 == 0 && (nst = conv_rows_stages(BN, 64, W, cin)) &&
                 conv_map<64>(X, Bn, H, W, cin, ldx, &m, true))
                 return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, sms, err, st);
@@ -1220,7 +1209,7 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
     if constexpr (BN % 64 == 0) {
         if (g_conv_tma && cin % 64 == 0 && 2 * GM * conv_ws_tiles(Bn, H, W) <= 3 * M &&
             conv_map<64>(X, Bn, H, W, cin, ldx, &m, true))
-            return conv_ws(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
+            return conv_ws(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, sms, err, st);
     }
     if (g_conv_tma && M % GM == 0) {   // box copies of the input when the shape tiles
         if (cin % 32 == 0 && conv_map<32>(X, Bn, H, W, cin, ldx, &m))
@@ -1709,14 +1698,9 @@ bool wgrad_rows_launch(const void* X, const void* Dz, float* work, int Bn, int H
     if (!strip_map<WC>(X, Bn, H, W, ldx, &xm) ||
         !strip_map<(BN % 64 == 0 ? 64 : (BN % 32 == 0 ? 32 : 16))>(Dz, Bn, H, W, ldz, &zm))
         return false;
-    static bool attr = false;
+    static PerDevice limit;
     *rc = XBG_ERR_CUDA;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_wgrad_rows<BN, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, WR_SMEM) !=
-            cudaSuccess)
-            return true;
-        attr = true;
-    }
+    if (!smem_limit(limit, k_wgrad_rows<BN, WC>, WR_SMEM)) return true;
     k_wgrad_rows<BN, WC><<<dim3((unsigned)(cin / WC), (unsigned)ksplit), 192,
                            (size_t)wgrad_rows_smem(BN, WC, NX), st>>>(
         xm, zm, work, H * nseg, nseg, chunks, per, NX, cin, ldp, bias_row, err);
@@ -1729,13 +1713,8 @@ int wgrad_launch(const void* X, const void* Dz, float* gw, float* gb, float* wor
                  int ldx, int ldz, int ldw, int ksplit, int accumulate, int* err, cudaStream_t st) {
     constexpr int STAGE = GM * GK * 2 + BN * GK * 2;
     const size_t smem = (size_t)CSTAGES * STAGE + 1024;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_wgrad_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess)
-            return XBG_ERR_CUDA;
-        attr = true;
-    }
+    static PerDevice limit;
+    if (!smem_limit(limit, k_wgrad_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
     const int Kc = 9 * cin;
     const int ldp = Kc + 8;
     const int bias_row = gb ? 1 : 0;
