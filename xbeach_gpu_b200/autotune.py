@@ -108,6 +108,14 @@ def _apply(target, setting, choice):
     return True
 
 
+def _distinct(target, settings):
+    """The settings to measure: those without a (phase, variant) pair that names
+    another variant's kernel again (the target's variant_alias), which a caller or
+    an earlier cache entry may still use."""
+    alias = getattr(target, "variant_alias", ())
+    return [s for s in settings if not any(pv in alias for pv in s)]
+
+
 def _settings(cached):
     """A cached setting as (phase, variant) pairs (entries are lists of pairs)."""
     return tuple((int(p), int(v)) for p, v in cached)
@@ -134,7 +142,7 @@ def tune_model(model, cache=None, reps=3, use_cache=True):
             _apply(model, _settings(db[key]), choice)
             continue
         best = None
-        for setting in settings:
+        for setting in _distinct(model, settings):
             trial = {}
             if not _apply(model, setting, trial):
                 continue
@@ -189,7 +197,7 @@ def tune(batch, cache=None, reps=3, shapes=None, use_cache=True):
             choice[shape] = cached[1]
             continue
         best = None
-        for setting in settings:
+        for setting in _distinct(batch, settings):
             trial = {}
             if not _apply(batch, setting, trial):   # not available for this batch
                 continue

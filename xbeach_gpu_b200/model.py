@@ -13,7 +13,7 @@ import os
 
 import numpy as np
 
-from .abi import FIELD, INT_FIELDS, Params, STATUS_NAMES, XBG_FP32
+from .abi import FIELD, INT_FIELDS, Params, STATUS_NAMES, XBG_FP32, XBG_PHASE_WAVE
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libxbg_b200.so")
@@ -115,8 +115,15 @@ def _ptr(a):
     return a.ctypes.data_as(C.c_void_p)
 
 
+# (phase, variant) pairs that name a smaller variant's kernel again: the rows pass
+# with box copies is one kernel under 1 and 2
+VARIANT_ALIAS = frozenset({(XBG_PHASE_WAVE, 2)})
+
+
 class Model:
     """One device-resident model (one xbg_handle)."""
+
+    variant_alias = VARIANT_ALIAS
 
     def __init__(self, params, precision=XBG_FP32, _handle=None):
         self.L = load()
@@ -282,8 +289,8 @@ class Model:
         return [(names[k].decode(), float(ms[k])) for k in range(n.value)]
 
     def set_variant(self, phase, variant):
-        """Kernel variant of a phase (XBG_PHASE_WAVE: 1 and 2 TMA tiles,
-        0 thread-copied tiles; XBG_PHASE_FLOW: 1 fused
+        """Kernel variant of a phase (XBG_PHASE_WAVE: 1 TMA tiles (2 is the same
+        kernel), 0 thread-copied tiles; XBG_PHASE_FLOW: 1 fused
         momentum pass, 0 two passes; XBG_PHASE_TILE: the pointwise passes in
         0 32 x 8 or 1 64 x 4 blocks)."""
         _check(self.L.xbg_set_kernel_variant(self.h, phase, variant), "set_kernel_variant")
@@ -303,6 +310,8 @@ class Batch:
     """n scenarios advanced together, one launch per kernel for all of them
     (xbg_batch_*).  batch.scenario(s) is a Model on the batch's handle s for
     fields, boundaries and time; advance() steps all of them."""
+
+    variant_alias = VARIANT_ALIAS
 
     def __init__(self, params_list, precision=XBG_FP32):
         self.L = load()
