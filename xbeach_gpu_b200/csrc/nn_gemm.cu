@@ -46,17 +46,16 @@ inline int current_device() {
     int dev = -1;
     return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
 }
-// a kernel's dynamic shared memory limit on the current device; false on an error
+// a kernel's dynamic shared memory limit on the current device dev; false on an error
 template <class K>
-bool smem_limit(PerDevice& d, K kernel, int bytes) {
-    return d.get(current_device(), [&] {
+bool smem_limit(PerDevice& d, int dev, K kernel, int bytes) {
+    return d.get(dev, [&] {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
     }) != 0;
 }
-// SMs of the current device, 0 on an error
-inline int sm_count() {
+// SMs of the device, 0 on an error
+inline int sm_count(int dev) {
     static PerDevice sms;
-    const int dev = current_device();
     return sms.get(dev, [&] {
         int n = 0;
         return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 0;
@@ -256,7 +255,7 @@ int gemm_launch(const void* A, const void* B, const float* bias, void* C, int M,
     constexpr int STAGE = GM * GK * 2 + BN * GK * 2;
     const size_t smem = (size_t)GSTAGES * STAGE + 1024;
     static PerDevice limit;
-    if (!smem_limit(limit, k_gemm_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
+    if (!smem_limit(limit, current_device(), k_gemm_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
     dim3 grid((M + GM - 1) / GM, ksplit);
     k_gemm_tc<BN><<<grid, 256, smem, st>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)B, bias, C, M, N, K, lda,
                                            ldb, ldc, flags, err);
@@ -677,11 +676,11 @@ bool conv_map(const void* X, int B, int H, int W, int cin, int ldx, CUtensorMap*
 
 template <int BN, int WC>
 int conv_tma_launch(const CUtensorMap& m, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
-                    int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
+                    int N, int Kp, int ldw, int ldy, int flags, int dev, int* err, cudaStream_t st) {
     constexpr int STAGE = GM * GK * 2 + BN * GK * 2;
     const size_t smem = (size_t)CSTAGES * STAGE + 1024;
     static PerDevice limit;
-    if (!smem_limit(limit, k_conv_tma<BN, WC>, (int)smem)) return XBG_ERR_CUDA;
+    if (!smem_limit(limit, dev, k_conv_tma<BN, WC>, (int)smem)) return XBG_ERR_CUDA;
     const long long M = (long long)Bn * H * W;
     k_conv_tma<BN, WC><<<(unsigned)((M + GM - 1) / GM), 256, smem, st>>>(m, (const __nv_bfloat16*)Wt, bias, Y, Bn,
                                                                           H, W, cin, N, Kp, ldw, ldy, flags, err);
@@ -982,9 +981,9 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
 
 template <int BN, int WC>
 int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
-                     int ldw, int ldy, int flags, int nst, int sms, int* err, cudaStream_t st) {
+                     int ldw, int ldy, int flags, int nst, int dev, int sms, int* err, cudaStream_t st) {
     static PerDevice limit;
-    if (!smem_limit(limit, k_conv_rows<BN, WC>, CR_SMEM)) return XBG_ERR_CUDA;
+    if (!smem_limit(limit, dev, k_conv_rows<BN, WC>, CR_SMEM)) return XBG_ERR_CUDA;
     const int S = Bn * ((W + GM - 1) / GM);
     const RowsRun run = conv_rows_run(S, H, sms, BN <= 32 || BN <= cin);
     k_conv_rows<BN, WC><<<(unsigned)conv_rows_ctas(run, S, H), CR_THREADS, (size_t)conv_rows_smem(BN, WC, cin, nst), st>>>(
@@ -1144,10 +1143,10 @@ inline long long conv_ws_tiles(int Bn, int H, int W) {
 
 template <int BN, int ST>
 int conv_ws_launch(const CUtensorMap& xm, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
-                   int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
+                   int N, int Kp, int ldw, int ldy, int flags, int dev, int* err, cudaStream_t st) {
     constexpr size_t smem = (size_t)ST * (GM + BN) * GK * 2 + 1024;
     static PerDevice limit;
-    if (!smem_limit(limit, k_conv_ws<BN, ST>, (int)smem)) return XBG_ERR_CUDA;
+    if (!smem_limit(limit, dev, k_conv_ws<BN, ST>, (int)smem)) return XBG_ERR_CUDA;
     CUtensorMap wm;
     if (!weight_map(Wt, N, Kp, ldw, BN, &wm)) return XBG_ERR_CUDA;
     const dim3 grid((unsigned)conv_ws_tiles(Bn, H, W), (unsigned)(N / BN));
@@ -1162,12 +1161,12 @@ int conv_ws_launch(const CUtensorMap& xm, const void* Wt, const float* bias, voi
 // stages 10.1; slices of 64 the same either way), else two with half of them (150
 // tiles 12.8, with deep stages 16.4).
 inline int conv_ws(const CUtensorMap& xm, const void* Wt, const float* bias, void* Y, int Bn, int H, int W, int cin,
-                   int N, int Kp, int ldw, int ldy, int flags, int sms, int* err, cudaStream_t st) {
+                   int N, int Kp, int ldw, int ldy, int flags, int dev, int sms, int* err, cudaStream_t st) {
     const long long tiles = conv_ws_tiles(Bn, H, W);
     const bool wide = N % 128 == 0 && tiles * (N / 64) > sms;
     const bool deep = tiles * (N / (wide ? 128 : 64)) <= sms;
 #define XBG_CONV_WS(BN, ST) \
-    conv_ws_launch<BN, ST>(xm, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st)
+    conv_ws_launch<BN, ST>(xm, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, dev, err, st)
     if (wide) return deep ? XBG_CONV_WS(128, 6) : XBG_CONV_WS(128, 3);
     return deep ? XBG_CONV_WS(64, 8) : XBG_CONV_WS(64, 4);
 #undef XBG_CONV_WS
@@ -1182,11 +1181,9 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
                 int N, int Kp, int ldw, int ldy, int flags, int* err, cudaStream_t st) {
     constexpr int STAGE = GM * GK * 2 + BN * GK * 2;
     const size_t smem = (size_t)CSTAGES * STAGE + 1024;
-    static PerDevice limit;
-    if (!smem_limit(limit, k_conv_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
     const long long M = (long long)Bn * H * W;
     CUtensorMap m;
-    const int sms = sm_count();
+    const int dev = current_device(), sms = sm_count(dev);
     if (!sms) return XBG_ERR_CUDA;
     if constexpr (BN <= 128) {
         // over rows where the weights fit beside the stages (the input is read three
@@ -1195,28 +1192,30 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
             int nst = 0;
             if (cin % 64 == 0 && (nst = conv_rows_stages(BN, 64, W, cin)) &&
                 conv_map<64>(X, Bn, H, W, cin, ldx, &m, true))
-                return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, sms, err, st);
+                return conv_rows_launch<BN, 64>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, dev, sms, err, st);
             if (cin % 32 == 0 && (nst = conv_rows_stages(BN, 32, W, cin)) &&
                 conv_map<32>(X, Bn, H, W, cin, ldx, &m, true))
-                return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, sms, err, st);
+                return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, dev, sms, err, st);
             if (cin % 32 != 0 && cin % 16 == 0 && conv_rows_pays(BN, 16, M, sms) &&
                 (nst = conv_rows_stages(BN, 16, W, cin)) &&
                 conv_map<16>(X, Bn, H, W, cin, ldx, &m, true))
-                return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, sms, err, st);
+                return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, dev, sms, err, st);
         }
     }
     // tile by tile in 64-channel chunks where the tiles lie inside the image for two thirds
     if constexpr (BN % 64 == 0) {
         if (g_conv_tma && cin % 64 == 0 && 2 * GM * conv_ws_tiles(Bn, H, W) <= 3 * M &&
             conv_map<64>(X, Bn, H, W, cin, ldx, &m, true))
-            return conv_ws(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, sms, err, st);
+            return conv_ws(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, dev, sms, err, st);
     }
     if (g_conv_tma && M % GM == 0) {   // box copies of the input when the shape tiles
         if (cin % 32 == 0 && conv_map<32>(X, Bn, H, W, cin, ldx, &m))
-            return conv_tma_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
+            return conv_tma_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, dev, err, st);
         if (cin % 32 != 0 && conv_map<16>(X, Bn, H, W, cin, ldx, &m))
-            return conv_tma_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, err, st);
+            return conv_tma_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, N, Kp, ldw, ldy, flags, dev, err, st);
     }
+    static PerDevice limit;
+    if (!smem_limit(limit, dev, k_conv_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
     k_conv_tc<BN><<<(unsigned)((M + GM - 1) / GM), 256, smem, st>>>((const __nv_bfloat16*)X,
                                                                      (const __nv_bfloat16*)Wt, bias, Y, Bn, H, W, cin,
                                                                      ldx, N, Kp, ldw, ldy, flags, err);
@@ -1689,7 +1688,7 @@ __global__ void __launch_bounds__(192, 1)
 // false where the shape does not fit (*rc unset), else launched with status *rc
 template <int BN, int WC>
 bool wgrad_rows_launch(const void* X, const void* Dz, float* work, int Bn, int H, int W, int cin, int ldx, int ldz,
-                       int ldp, int bias_row, int ksplit, int* err, cudaStream_t st, int* rc) {
+                       int ldp, int bias_row, int ksplit, int dev, int* err, cudaStream_t st, int* rc) {
     const int nseg = W / WR_P, chunks = Bn * H * nseg, per = (chunks + ksplit - 1) / ksplit;
     // the rows around a run are copied too, so a run is at least as long as they are
     const int NX = wgrad_rows_slots(BN, WC, nseg);
@@ -1700,7 +1699,7 @@ bool wgrad_rows_launch(const void* X, const void* Dz, float* work, int Bn, int H
         return false;
     static PerDevice limit;
     *rc = XBG_ERR_CUDA;
-    if (!smem_limit(limit, k_wgrad_rows<BN, WC>, WR_SMEM)) return true;
+    if (!smem_limit(limit, dev, k_wgrad_rows<BN, WC>, WR_SMEM)) return true;
     k_wgrad_rows<BN, WC><<<dim3((unsigned)(cin / WC), (unsigned)ksplit), 192,
                            (size_t)wgrad_rows_smem(BN, WC, NX), st>>>(
         xm, zm, work, H * nseg, nseg, chunks, per, NX, cin, ldp, bias_row, err);
@@ -1713,8 +1712,7 @@ int wgrad_launch(const void* X, const void* Dz, float* gw, float* gb, float* wor
                  int ldx, int ldz, int ldw, int ksplit, int accumulate, int* err, cudaStream_t st) {
     constexpr int STAGE = GM * GK * 2 + BN * GK * 2;
     const size_t smem = (size_t)CSTAGES * STAGE + 1024;
-    static PerDevice limit;
-    if (!smem_limit(limit, k_wgrad_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
+    const int dev = current_device();
     const int Kc = 9 * cin;
     const int ldp = Kc + 8;
     const int bias_row = gb ? 1 : 0;
@@ -1722,12 +1720,14 @@ int wgrad_launch(const void* X, const void* Dz, float* gw, float* gb, float* wor
     bool rows = false;
     if constexpr (BN <= 128) {   // box copies where the shape tiles
         if (g_conv_tma && W % WR_P == 0 && cin % 32 == 0)
-            rows = wgrad_rows_launch<BN, 32>(X, Dz, work, Bn, H, W, cin, ldx, ldz, ldp, bias_row, ksplit, err, st, &rc);
+            rows = wgrad_rows_launch<BN, 32>(X, Dz, work, Bn, H, W, cin, ldx, ldz, ldp, bias_row, ksplit, dev, err, st, &rc);
         else if (g_conv_tma && W % WR_P == 0 && cin % 16 == 0)
-            rows = wgrad_rows_launch<BN, 16>(X, Dz, work, Bn, H, W, cin, ldx, ldz, ldp, bias_row, ksplit, err, st, &rc);
+            rows = wgrad_rows_launch<BN, 16>(X, Dz, work, Bn, H, W, cin, ldx, ldz, ldp, bias_row, ksplit, dev, err, st, &rc);
     }
     if (rc != XBG_OK) return rc;
     if (!rows) {
+        static PerDevice limit;
+        if (!smem_limit(limit, dev, k_wgrad_tc<BN>, (int)smem)) return XBG_ERR_CUDA;
         dim3 grid((unsigned)((Kc + bias_row + GM - 1) / GM), (unsigned)ksplit);
         k_wgrad_tc<BN><<<grid, 256, smem, st>>>((const __nv_bfloat16*)X, (const __nv_bfloat16*)Dz, work, Bn, H, W,
                                                 cin, ldx, ldz, ldp, bias_row, err);
