@@ -1,5 +1,5 @@
 """The warp-specialised convolutions -- over rows of 128 pixels (layers whose
-weights fit in shared memory, W a multiple of 128) and tile by tile (64 input
+weights fit in shared memory, W from 128 on) and tile by tile (64 input
 channels at a time) -- against the thread-gathered convolution: the same
 products in the same order, so the outputs are equal bit for bit.  Shapes: one
 row per CTA and fewer rows than SMs, runs that cross strips and images, one row

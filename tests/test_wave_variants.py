@@ -1,12 +1,12 @@
-"""Kernel variants of the same arithmetic.  The wave rows pass has three:
+"""Kernel variants of the same arithmetic.  The wave rows pass has two:
 plane tiles moved by the tensor memory accelerator (one box copy per bin,
-issued by one thread; the default where it applies) with one or with two
-cells per thread, and plane tiles copied by every thread (cp.async).  The
+issued by one thread; the default where it applies, under the numbers 1 and
+2), and plane tiles copied by every thread (cp.async).  The
 flow step's momentum updates run as one pass (uu* of the tile and its ring
 in shared memory) or as two.  The passes that read only a cell and its
 nearest neighbours run in 32 x 8 or 64 x 4 blocks.  Each must give the same
 state bit for bit over whole coupled steps, on grids whose tiles are partial in x and in y, at the
-offshore and lateral edges, for few bins (fewer than the four tile buffers),
+offshore and lateral edges, for few bins (fewer than the six tile buffers),
 with and without the roller, in FP32 and FP64."""
 import numpy as np
 import pytest

@@ -362,8 +362,8 @@ __device__ __forceinline__ void b_flow_v(const Dev<R>& S, const Konst<R>& K, con
     if (off) return;
     S.tmp[T_VV][IDX(ix, iy)] = v;
 }
-// batched: 64 registers instead of 78, 43.0 -> 32.8 us over ten domains of 128 x 64 to
-// 1024 x 512 (flow_u so bounded spills: 30.7 -> 34.8)
+// batched: 64 registers (4 bytes spilled) instead of 78, 43.0 -> 32.8 us over ten domains
+// of 128 x 64 to 1024 x 512; flow_u takes 64 without a bound
 XBG_KERNELS_B(flow_v, 4)
 
 // flow_u and flow_v in one pass.  eulervstep reads uu* at the cell, its left,

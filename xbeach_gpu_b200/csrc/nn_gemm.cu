@@ -1005,7 +1005,7 @@ int conv_rows_launch(const CUtensorMap& m, const void* Wt, const float* bias, vo
 // k_conv_tma: 256 -> 256 channels at 64 x 128 pixels 50 -> 14 us, 384 -> 128 at
 // 128 x 256 69 -> 27, 192 -> 64 at 256 x 512 94 -> 47.
 // With ragged tiles (and strips in k_conv_rows) instead of the gathered path, a
-// prediction of 240 x 1016 pixels takes 328 instead of 623 us, of 128 x 200 221 of 346.
+// prediction of 240 x 1016 pixels takes 323 instead of 636 us, of 128 x 200 215 of 348.
 template <int BN, int ST>
 __global__ void __launch_bounds__(192, 1)
     k_conv_ws(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,

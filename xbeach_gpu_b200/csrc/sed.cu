@@ -293,7 +293,7 @@ __device__ __forceinline__ void b_sed_b(const Dev<R>& S, const Konst<R>& K, cons
         S.tmp[T_STDEP][i] = sd0 - dzg;
     }
 }
-// batched: 64 registers instead of 80, 49.2 -> 45.1 us over ten domains
+// batched: 64 registers (68 bytes spilled) instead of 80, 49.2 -> 45.1 us over ten domains
 XBG_KERNELS_B(sed_b, 4)
 
 // zblatbnd source cell (Sediment_kernel.cu:970-1018, pre-kernel reads)

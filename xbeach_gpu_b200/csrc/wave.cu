@@ -159,8 +159,8 @@ __device__ __forceinline__ R flux2(R qm2, R qm, R qi, R qp, R qp2, R cf, R cfmin
 // dt / dx (kin, kmin: the face speeds 0.5 (cg_i + cg_j) dt / dx), so a bin's
 // x or y flux difference is cos (sin) times fk(), and its Euler update
 // A = e - (cos fk_x + sin fk_y + dt / dtheta (theta-face difference)).  The
-// upwind side is the one of cos (sin): pos.  Both rows-pass kernels use
-// these two (bit-identical results).
+// upwind side is the one of cos (sin): pos.  The box-fed rows pass evaluates the
+// same expressions on pairs of cells (xy_flux; bit-identical results).
 template <class R>
 __device__ __forceinline__ R flux2kv(R qm2, R qm, R qi, R qp, R qp2, bool pos, R kin, R kmin) {
     const R ain = upw(pos ? qi : qp, pos ? qm : qp2);
