@@ -1,8 +1,7 @@
 """The convolution and the weight gradient where every SM has work and each block
-many rows (more than accumulator slots), several launches in a row, against the
-thread-gathered kernels, bit for bit: every output width of the kernel over rows
-whose blocks ask for all tensor memory columns, and the widths that are left to
-the other kernels because two such blocks would fit on an SM."""
+many rows (more than stages and accumulator slots hold), several launches in a row,
+against the thread-gathered kernels, bit for bit: output widths whose blocks ask for
+all tensor memory columns, and the widths that are left to the other kernels."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -25,7 +24,15 @@ def test_conv_runs(B, H, W, cin, N):
     _conv(B, H, W, cin, N)
 
 
-def _conv(B, H, W, cin, N):
+# blocks whose stores take as long as their products, so that the product warp waits for accumulators
+@pytest.mark.parametrize("B,H,W,cin,N", [(5, 64, 455, 64, 128), (4, 256, 256, 32, 128), (3, 194, 513, 32, 96),
+                                         (5, 117, 512, 32, 64)])
+def test_conv_stores_bound(B, H, W, cin, N):
+    import torch
+    _conv(B, H, W, cin, N, torch.float32)
+
+
+def _conv(B, H, W, cin, N, out=None):
     import torch
     from xbeach_gpu_b200 import surrogate as sg
     g = torch.Generator(device="cuda").manual_seed(cin + N)
@@ -35,7 +42,7 @@ def _conv(B, H, W, cin, N):
     w = torch.zeros(N, Kp, device="cuda")
     w[:, :9 * cin] = torch.randn(N, 9 * cin, device="cuda", generator=g) / (9 * cin) ** 0.5
     w = w.to(torch.bfloat16)
-    y = [torch.zeros(P, N, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    y = [torch.zeros(P, N, device="cuda", dtype=out or torch.bfloat16) for _ in range(2)]
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     for on in (0, 1):
         assert L.xbg_nn_conv_set_tma(on) == 0

@@ -1,8 +1,7 @@
-"""What the box-fed convolution and weight-gradient kernels ask of an SM, over
-every channel count and width that they take: no mix of CTAs whose shared memory
-fits on an SM -- of these kernels and of the other tensor-core kernels, as launches
-on several streams put them together -- asks for more than its 512 tensor memory
-columns, so that no allocation waits."""
+"""What the box-fed convolution and weight-gradient kernels ask of an SM, over every
+channel count and width that they take: shared memory within a block's limit, no
+more blocks of a launch on an SM than its 512 tensor memory columns serve, a stage
+for every box of a row, and runs of rows that cover the image once."""
 import ctypes as C
 import os
 import subprocess
@@ -52,17 +51,22 @@ def test_plans_fit_a_block(plan):
         assert 1024 + n * 512 * wc + 384 * bn <= plan.wgrad_smem(bn, wc, n) <= CTA_MAX - 512
 
 
-def test_no_mix_of_blocks_exceeds_tensor_memory(plan):
-    items = {(plan.rows_smem(bn, wc, cin, n) + 1024, plan.rows_cols(bn)) for bn, wc, cin, n in _rows(plan)}
-    items |= {(plan.wgrad_smem(bn, wc, n) + 1024, plan.wgrad_cols(bn)) for bn, wc, n in _wgrad(plan)}
-    # the gathered kernels and the tiled one: stages of 64 channels of 128 pixels and of the weights
-    for bn in WIDTHS + (192, 256):
-        items.add((3 * 128 * (128 + bn) + 2048, max(32, 1 << (bn - 1).bit_length())))
-    items |= {(st * 128 * (128 + bn) + 2048, bn) for bn, st in ((128, 6), (128, 3), (64, 8), (64, 4))}
-    best = [0] * (SM // 256 + 1)   # most columns in this much shared memory
-    for s in range(1, len(best)):
-        best[s] = max([best[s - 1]] + [best[s - b // 256] + c for b, c in items if b // 256 <= s])
-    assert best[-1] <= COLS
+def test_blocks_on_an_sm_fit_its_tensor_memory(plan):
+    """As many blocks of a launch as an SM's shared memory holds ask for no more than
+    its columns, so that none is placed there only to wait."""
+    for bn, wc, cin, n in _rows(plan):
+        assert SM // (plan.rows_smem(bn, wc, cin, n) + 1024) * plan.rows_cols(bn) <= COLS, (bn, wc, cin)
+    for bn, wc, n in _wgrad(plan):
+        assert SM // (plan.wgrad_smem(bn, wc, n) + 1024) * plan.wgrad_cols(bn) <= COLS, (bn, wc, n)
+
+
+def test_layers_left_to_the_other_kernels(plan):
+    """16-channel boxes with more output than input channels, beyond 32."""
+    took = {(cin, bn) for bn, wc, cin, n in _rows(plan)}
+    for cin, bn in ((16, 48), (16, 64), (16, 96), (16, 128), (48, 64), (48, 96), (48, 128), (80, 96), (80, 128)):
+        assert (cin, bn) not in took
+    for cin, bn in ((16, 16), (16, 32), (32, 128), (48, 48), (64, 128), (80, 64), (96, 32)):
+        assert (cin, bn) in took
 
 
 def test_a_rows_boxes_have_stages(plan):

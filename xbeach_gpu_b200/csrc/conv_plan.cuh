@@ -12,8 +12,6 @@ namespace xbg {
 namespace nn {
 
 constexpr int PLAN_GM = 128;               // pixels of a strip
-constexpr int SM_SMEM = 228 * 1024;        // shared memory of an SM; a CTA takes 1 KB beside its own
-constexpr int SM_TCOLS = 512;              // tensor memory columns of an SM
 constexpr int CR_MAXST = 18;               // input stages of k_conv_rows at most
 constexpr int CR_SMEM = 225 * 1024;        // its dynamic shared memory at most
 constexpr int WR_P = 64;                   // pixels of a chunk of k_wgrad_rows
@@ -21,13 +19,10 @@ constexpr int WR_MX = 24;                  // its input slots at most
 constexpr int WR_ND = 3;                   // its dz slots
 constexpr int WR_SMEM = 226 * 1024;
 
-// CTAs on an SM may not ask for more than its columns together: a CTA whose
-// allocation has to wait for another's columns faulted (16 -> 128 channels at
-// 4 x 256 x 256: 512 columns with 109 KB of shared memory, so two CTAs to an SM).
-// So every CTA takes at least the share of shared memory that it takes of the
-// columns, whatever kernels meet on an SM: this many bytes, less what a kernel
-// keeps in static shared memory.
-XBG_PLAN int tcols_smem(int cols) { return SM_SMEM / SM_TCOLS * cols - 2048; }
+// Where a CTA asks for more than half of an SM's 512 tensor memory columns it takes
+// more than half of the shared memory too: a second CTA of the launch would be
+// placed there only to wait for columns.
+constexpr int HALF_TCOLS = 256, HALF_SMEM = 115 * 1024;
 XBG_PLAN int at_least(int a, int b) { return a > b ? a : b; }
 
 // ---- k_conv_rows
@@ -40,14 +35,17 @@ XBG_PLAN int conv_rows_bytes(int bn, int wc, int cin, int nst) {
     return 1024 + nst * PLAN_GM * wc * 2 + 9 * cin * bn * 2;
 }
 XBG_PLAN int conv_rows_smem(int bn, int wc, int cin, int nst) {
-    const int share = tcols_smem(conv_rows_cols(bn));
-    return at_least(conv_rows_bytes(bn, wc, cin, nst), share < CR_SMEM ? share : CR_SMEM);
+    return at_least(conv_rows_bytes(bn, wc, cin, nst), conv_rows_cols(bn) > HALF_TCOLS ? HALF_SMEM : 0);
 }
 // stages that fit beside the weights of a layer (0: k_conv_rows does not apply)
 XBG_PLAN int conv_rows_stages(int bn, int wc, int W, int cin) {
     // the last strip of a row may be ragged; strips of which over a third lies outside the image are not worth it
     const int strips = (W + PLAN_GM - 1) / PLAN_GM;
     if (bn > 128 || W < PLAN_GM || 2 * strips * PLAN_GM > 3 * W) return 0;
+    // 16-channel boxes with more output channels (beyond 32) than input channels are
+    // left to the other kernels: 16 -> 128 and 48 -> 96 faulted before whole warps
+    // waited, and it is not shown that those waits were all that was wrong there
+    if (wc == 16 && bn > 32 && bn > cin) return 0;
     const int nb = 3 * (cin / wc);   // an input row's boxes are waited for together; two rows' worth, or nearly
     if (nb > 30) return 0;
     const int room = CR_SMEM - conv_rows_bytes(bn, wc, cin, 0), box = PLAN_GM * wc * 2;
@@ -55,9 +53,6 @@ XBG_PLAN int conv_rows_stages(int bn, int wc, int W, int cin) {
     if (n < nb + (nb + 1) / 2) return 0;
     const int nst = n > CR_MAXST ? CR_MAXST : n;
     if (nst < nb) return 0;
-    // 512 columns in a CTA that needs less than half of the SM's shared memory (16
-    // input channels, 48 to 128 output channels): left to the other kernels
-    if (2 * conv_rows_cols(bn) > SM_TCOLS && 2 * (conv_rows_bytes(bn, wc, cin, nst) + 1024) <= SM_SMEM) return 0;
     return nst;
 }
 // 16-channel boxes (32 bytes a pixel) pay from three rows a CTA on, with 16 output
@@ -101,8 +96,7 @@ XBG_PLAN int wgrad_rows_cols(int bn) { return bn <= 16 ? 64 : (bn <= 32 ? 128 : 
 XBG_PLAN int wgrad_rows_fixed(int bn, int wc) { return 1024 + (wc == 16 ? 4 * WR_P * wc * 2 : 0) + WR_ND * WR_P * bn * 2; }
 XBG_PLAN int wgrad_rows_bytes(int bn, int wc, int nx) { return wgrad_rows_fixed(bn, wc) + nx * 4 * WR_P * wc * 2; }
 XBG_PLAN int wgrad_rows_smem(int bn, int wc, int nx) {
-    const int share = tcols_smem(wgrad_rows_cols(bn));
-    return at_least(wgrad_rows_bytes(bn, wc, nx), share < WR_SMEM ? share : WR_SMEM);
+    return at_least(wgrad_rows_bytes(bn, wc, nx), wgrad_rows_cols(bn) > HALF_TCOLS ? HALF_SMEM : 0);
 }
 // input slots of rows of nseg chunks: the resident chunks and two to four copies
 // ahead (0: k_wgrad_rows does not apply)
@@ -111,8 +105,6 @@ XBG_PLAN int wgrad_rows_slots(int bn, int wc, int nseg) {
     if (nx > 2 * nseg + 5) nx = 2 * nseg + 5;
     if (nx > WR_MX) nx = WR_MX;
     if (nx < 2 * nseg + 3) return 0;
-    // as for k_conv_rows (16-channel boxes, 96 output channels, rows of one chunk)
-    if (2 * wgrad_rows_cols(bn) > SM_TCOLS && 2 * (wgrad_rows_bytes(bn, wc, nx) + 1024) <= SM_SMEM) return 0;
     return nx;
 }
 // Where it pays: 32-channel boxes; 16-channel boxes for 16 input channels, and for

@@ -15,13 +15,10 @@
 namespace xbg {
 namespace nn {
 
-// The last copy into `slot`, -1 if there was none: copies 0 .. n-1 were issued,
-// and of the group of copies n, n+1, ... that was under way, those whose bits
-// are set in `some` (the group holds fewer copies than there are slots).
-XBG_RING_HD int ring_last(int n, unsigned some, int slots, int slot) {
-    int c = slot - n % slots;   // the group's copy into this slot
+// The last of the copies 0 .. n-1 into `slot`, -1 if there was none.
+XBG_RING_HD int ring_last(int n, int slots, int slot) {
+    int c = slot - n % slots;   // copy n + c is the slot's next one
     if (c < 0) c += slots;
-    if (c < 32 && (some >> c & 1u)) return n + c;
     return n + c - slots < 0 ? -1 : n + c - slots;
 }
 // ... and the parity of the phase that it completes

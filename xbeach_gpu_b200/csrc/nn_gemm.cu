@@ -699,23 +699,28 @@ __device__ __forceinline__ bool role_wait(unsigned a, unsigned parity, int* bad)
     *(volatile int*)bad = 1;
     return false;
 }
+// ... by a whole warp, for one barrier: the same answer in every lane, and the lanes
+// together again.  A role issues its copies and products from one lane of a warp
+// that runs in step: their operands go through registers that the warp's lanes share,
+// so no other lane may be somewhere else in the code meanwhile (a lane that leaves
+// the wait one poll before another, or a time-out's way out of the loop).
+__device__ __forceinline__ bool warp_wait(unsigned a, unsigned parity, int* bad) {
+    return __all_sync(0xffffffffu, role_wait(a, parity, bad));
+}
 // Leaving early: the last copy into each of a ring's slots lands first, a lane per
-// slot (bounded).  n and `some` as in ring_last, the same in every lane.
-__device__ __forceinline__ void drain_copies(unsigned long long* full, int slots, int n, unsigned some, int lane) {
+// slot (bounded).  n as in ring_last, the same in every lane.
+__device__ __forceinline__ void drain_copies(unsigned long long* full, int slots, int n, int lane) {
     if (lane < slots) {
-        const int q = ring_last(n, some, slots, lane);
+        const int q = ring_last(n, slots, lane);
         if (q >= 0) mbar_wait(smem_u32(&full[lane]), ring_parity(q, slots));
     }
     __syncwarp();
-}
-// the value of the lane that issues (each lane counts its own way through the loop)
-__device__ __forceinline__ int of_leader(int v, unsigned leader) {
-    return __shfl_sync(0xffffffffu, v, __ffs((int)__ballot_sync(0xffffffffu, leader != 0)) - 1);
 }
 // CW accumulator columns of this warp's 32 tensor-memory lanes (one pixel per
 // lane) in registers
 template <int CW>
 __device__ __forceinline__ void load_cols(unsigned (&v)[CW], unsigned taddr) {
+    __syncwarp();   // an aligned instruction: the whole warp, also after a store by some of its lanes
 #pragma unroll
     for (int h = 0; h < CW; h += 8)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
@@ -831,7 +836,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
     const unsigned tmem = tmem_slot;
     unsigned leader;   // one lane of each warp
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
-    auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
+    auto wait = [&](unsigned a, unsigned parity) -> bool { return warp_wait(a, parity, &bad); };
     // The run's segments (rows of one strip of one image) in order:
     // seg(b, x0, y0, n, o0) with o0 the number of the segment's first row in
     // the run; returns false to stop.
@@ -842,8 +847,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
             l += n;
         }
     };
-    int sent = 0;        // copies issued, in whole rows; of the row a wait ended, the lanes that issued
-    unsigned some = 0;
+    int sent = 0;   // copies issued
     // one lane's commit covers what it issued before
     auto commit = [&](const void* bar) {
         if (leader) asm volatile(
@@ -851,37 +855,28 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
             : "memory");
     };
     if (warp == 0) {
-        // ---- copies: lane c takes box c of an input row (dx, channel group)
-        const int cx = lane / ncg - 1, cch = lane % ncg * WC;
-        int s = 0;   // the row's first stage
+        // ---- copies: the boxes of an input row in the order (dx, channel group)
+        int s = 0;
         unsigned ph = 0;
         segments([&](int b, int x0, int y0, int n, int) {
-            for (int r = y0 - 1; r <= y0 + n; r++) {
-                bool ok = true;
-                if (lane < nb) {
-                    const int t = s + lane < nst ? s + lane : s + lane - nst;
-                    const unsigned tp = s + lane < nst ? ph : ph ^ 1u;
-                    ok = wait(smem_u32(&empty[t]), tp ^ 1u);
-                    if (ok) {
-                        const unsigned fb = smem_u32(&full[t]);
+            for (int r = y0 - 1; r <= y0 + n; r++)
+                for (int c = 0, x = x0 - 1, ch = 0; c < nb; c++) {
+                    if (!wait(smem_u32(&empty[s]), ph ^ 1u)) return false;
+                    if (leader) {
+                        const unsigned fb = smem_u32(&full[s]);
                         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb),
                                      "r"((unsigned)BOX)
                                      : "memory");
                         asm volatile(
                             "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                            "[%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(base + (unsigned)t * BOX),
-                            "l"((unsigned long long)&xmap), "r"(cch), "r"(x0 + cx), "r"(r), "r"(b), "r"(fb)
+                            "[%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(base + (unsigned)s * BOX),
+                            "l"((unsigned long long)&xmap), "r"(ch), "r"(x), "r"(r), "r"(b), "r"(fb)
                             : "memory");
                     }
+                    sent++;
+                    if (++s == nst) { s = 0; ph ^= 1u; }
+                    if ((ch += WC) == cin) { ch = 0; x++; }
                 }
-                if (!__all_sync(0xffffffffu, ok)) {
-                    some = __ballot_sync(0xffffffffu, ok && lane < nb);
-                    return false;
-                }
-                sent += nb;
-                s += nb;
-                if (s >= nst) { s -= nst; ph ^= 1u; }
-            }
             return true;
         });
     } else if (warp == 1) {   // ---- products: the warp runs in step, one lane issues
@@ -900,25 +895,19 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
             for (int r = y0 - 1; r <= y0 + n; r++) {
                 const int on = o0 + r + 1 - y0;   // the output row that starts here, if any
                 const bool v0 = r + 1 < y0 + n, v1 = r >= y0 && r < y0 + n, v2 = r - 1 >= y0;
-                // the row's boxes and, for the row that starts, its accumulator: one
-                // lane waits for each
-                bool ok = true;
-                if (lane < nb)
-                    ok = wait(smem_u32(&full[s + lane < nst ? s + lane : s + lane - nst]), s + lane < nst ? ph : ph ^ 1u);
-                else if (lane == 31 && v0)
-                    ok = wait(smem_u32(&aempty[on % NS]), ((unsigned)(on / NS) & 1u) ^ 1u);
-                if (!__all_sync(0xffffffffu, ok)) return false;
-                tc_fence_after();
+                // the accumulator of the row that starts here
+                if (v0 && !wait(smem_u32(&aempty[on % NS]), ((unsigned)(on / NS) & 1u) ^ 1u)) return false;
                 // accumulators of the output rows that see this input row as tap row 0, 1, 2
                 const unsigned d0 = tmem + (unsigned)((on + NS) % NS) * STRIDE, d1 = tmem + (unsigned)((on - 1 + NS) % NS) * STRIDE,
                                d2 = tmem + (unsigned)((on - 2 + NS) % NS) * STRIDE;
                 // dx, channel group; inner: all three output rows exist
-                auto boxes = [&](auto inner) {
+                auto boxes = [&](auto inner) -> bool {
                     constexpr bool IN = decltype(inner)::value;
                     uint64_t db = db0;
-                    int t = s;
                     for (int c = 0; c < nb; c++) {
-                        const uint64_t da = da0 + (uint64_t)((unsigned)t * BOX >> 4);
+                        if (!wait(smem_u32(&full[s]), ph)) return false;
+                        tc_fence_after();
+                        const uint64_t da = da0 + (uint64_t)((unsigned)s * BOX >> 4);
 #pragma unroll
                         for (int j = 0; j < WC / 16; j++) {
                             // the row that starts here: its first product overwrites
@@ -926,15 +915,13 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
                             if (IN || v1) mma(d1, da + 2 * j, db + tstep + 2 * j, 1u);
                             if (IN || v2) mma(d2, da + 2 * j, db + 2 * tstep + 2 * j, 1u);
                         }
-                        commit(&empty[t]);
+                        commit(&empty[s]);
                         db += CHUNK >> 4;
-                        if (++t == nst) t = 0;
+                        if (++s == nst) { s = 0; ph ^= 1u; }
                     }
+                    return true;
                 };
-                if (v0 && v1 && v2) boxes(std::true_type{});
-                else boxes(std::false_type{});
-                s += nb;
-                if (s >= nst) { s -= nst; ph ^= 1u; }
+                if (!(v0 && v1 && v2 ? boxes(std::true_type{}) : boxes(std::false_type{}))) return false;
                 if (v2) commit(&afull[(on - 2 + NS) % NS]);   // output row r-1 has all its taps
             }
             return true;
@@ -944,7 +931,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
         segments([&](int b, int x0, int y0, int n, int o0) {
             for (int y = y0; y < y0 + n; y++) {
                 const int o = o0 + y - y0, slot = o % NS;
-                if (!__all_sync(0xffffffffu, wait(smem_u32(&afull[slot]), (unsigned)(o / NS) & 1u))) return false;
+                if (!wait(smem_u32(&afull[slot]), (unsigned)(o / NS) & 1u)) return false;
                 tc_fence_after();
                 const size_t row = (size_t)(b * H + y) * W + x0 + q * 32 + lane;
                 constexpr int CW = BN % 32 == 0 ? 32 : 16;   // columns at a time
@@ -967,7 +954,7 @@ __global__ void __launch_bounds__(CR_THREADS, 1)
     }
     __syncthreads();   // every role has ended: `bad` is final
     if (bad) {         // a wait ran out: copies and products in flight end before shared and tensor memory go
-        if (warp == 0) drain_copies(full, nst, sent, some, lane);
+        if (warp == 0) drain_copies(full, nst, sent, lane);
         if (warp == 1) {
             commit(&drain);
             mbar_wait(smem_u32(&drain), 0);
@@ -1038,7 +1025,7 @@ __global__ void __launch_bounds__(192, 1)
     const unsigned tmem = tmem_slot;
     unsigned leader;   // one lane of each warp
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
-    auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
+    auto wait = [&](unsigned a, unsigned parity) -> bool { return warp_wait(a, parity, &bad); };
     int sent = 0;   // chunks whose copies were issued
     if (warp == 0) {   // ---- copies
         const unsigned bytes = (unsigned)(R * Wt) * GK * 2 + B_BYTES;
@@ -1098,7 +1085,7 @@ __global__ void __launch_bounds__(192, 1)
                          : "memory");
     } else {   // ---- the tile out
         const int q = warp & 3;
-        if (__all_sync(0xffffffffu, wait(smem_u32(&done), 0)) && !*(volatile int*)&bad) {
+        if (wait(smem_u32(&done), 0) && __all_sync(0xffffffffu, !*(volatile int*)&bad)) {
             tc_fence_after();
             const int p = q * 32 + lane, r = p / Wt, x = x0 + p - r * Wt, y = y0 + r;
             const size_t row = (size_t)(b * H + y) * W + x;
@@ -1113,10 +1100,7 @@ __global__ void __launch_bounds__(192, 1)
     }
     __syncthreads();   // every role has ended: `bad` is final
     if (bad) {         // as in k_conv_rows
-        if (warp == 0) {
-            __syncwarp();
-            drain_copies(full, ST, of_leader(sent, leader), 0, lane);
-        }
+        if (warp == 0) drain_copies(full, ST, sent, lane);
         if (warp == 1) mbar_wait(smem_u32(&done), 0);
         if (tid == 0) atomicExch(err, XBG_ERR_TIMEOUT);
     }
@@ -1550,7 +1534,7 @@ __global__ void __launch_bounds__(192, 1)
     const unsigned tmem = tmem_slot;
     unsigned leader;   // one lane of each warp
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
-    auto wait = [&](unsigned a, unsigned parity) -> bool { return role_wait(a, parity, &bad); };
+    auto wait = [&](unsigned a, unsigned parity) -> bool { return warp_wait(a, parity, &bad); };
     int nxl = 0, nzl = 0;   // input and dz chunks whose copies were issued
     if (warp == 0) {   // ---- copies: per image of the run, input chunks i0 - nseg .. i1 - 1 + nseg, dz chunks i0 .. i1 - 1
         auto box = [&](unsigned dst, const CUtensorMap* m, int c, int x, int y, int b, unsigned bar) {
@@ -1647,7 +1631,7 @@ __global__ void __launch_bounds__(192, 1)
         commit(&done);   // every product issued so far
     } else {   // ---- accumulator row m of y offset dy: x offset m / WC, channel m % WC
         const int q = warp & 3;
-        if (__all_sync(0xffffffffu, wait(smem_u32(&done), 0)) && !*(volatile int*)&bad) {
+        if (wait(smem_u32(&done), 0) && __all_sync(0xffffffffu, !*(volatile int*)&bad)) {
             tc_fence_after();
             const int m = q * 32 + lane, box = m / WC, ch = m - box * WC;
             float* dst = part + (size_t)blockIdx.y * BN * ldp;
@@ -1672,9 +1656,8 @@ __global__ void __launch_bounds__(192, 1)
     __syncthreads();   // every role has ended: `bad` is final
     if (bad) {         // as in k_conv_rows
         if (warp == 0) {
-            __syncwarp();
-            drain_copies(xfull, NX, of_leader(nxl, leader), 0, lane);
-            drain_copies(zfull, ND, of_leader(nzl, leader), 0, lane);
+            drain_copies(xfull, NX, nxl, lane);
+            drain_copies(zfull, ND, nzl, lane);
         }
         if (warp == 1) mbar_wait(smem_u32(&done), 0);
         if (tid == 0) atomicExch(err, XBG_ERR_TIMEOUT);
