@@ -5,6 +5,7 @@ extern "C" {
 int rows_stages(int bn, int wc, int W, int cin) { return conv_rows_stages(bn, wc, W, cin); }
 int rows_smem(int bn, int wc, int cin, int nst) { return conv_rows_smem(bn, wc, cin, nst); }
 int rows_cols(int bn) { return conv_rows_cols(bn); }
+int rows_pays(int bn, int cin, int W, int pixels, int sms) { return conv_rows_pays(bn, cin, W, pixels, sms); }
 int rows_run(int S, int H, int sms, int extra, int* lohi) {   // CTAs; [lo, hi) of each
     const RowsRun r = conv_rows_run(S, H, sms, extra != 0);
     const int n = conv_rows_ctas(r, S, H);

@@ -100,3 +100,14 @@ def test_runs_cover_every_row_once(plan, extra):
                 assert max(b - a for a, b in runs) <= per + extra
     buf = (C.c_int * 296)()
     assert plan.rows_run(2, 160, 148, 0, buf) == 108 and (buf[2], buf[3]) == (3, 6) and (buf[108], buf[109]) == (160, 163)
+
+
+# 16-channel boxes where the other kernels are the faster (a first size that pays is
+# beside each): too few rows a block, 16 outputs of 48 or 80 channels, wide strip edges
+@pytest.mark.parametrize("bn,cin,W,H,pays", [
+    (16, 16, 384, 256, 0), (16, 16, 512, 256, 0), (16, 16, 512, 336, 1), (32, 16, 240, 200, 0), (32, 16, 256, 256, 1),
+    (32, 16, 320, 200, 1), (32, 16, 344, 240, 1), (16, 48, 512, 256, 0), (16, 80, 1024, 512, 0), (48, 48, 344, 240, 0),
+    (48, 48, 300, 304, 0), (48, 48, 512, 256, 1), (32, 48, 192, 768, 0), (32, 80, 400, 400, 0), (32, 80, 512, 336, 1),
+    (16, 32, 128, 1, 1), (128, 64, 128, 1, 1)])
+def test_narrow_boxes_where_they_pay(plan, bn, cin, W, H, pays):
+    assert plan.rows_pays(bn, cin, W, H * W, 148) == pays

@@ -55,13 +55,20 @@ XBG_PLAN int conv_rows_stages(int bn, int wc, int W, int cin) {
     if (nst < nb) return 0;
     return nst;
 }
-// 16-channel boxes (32 bytes a pixel) pay from three rows a CTA on, with 16 output
-// channels from four: below, k_conv_tma's and k_conv_tc's blocks, two and more to an
-// SM, end first.  16 -> 32 channels at 128 x 128 pixels 5.5 us there, 6.5 here, at
-// 208 x 256 7.6, 8.4, at 256 x 256 10.5, 9.0; 48 -> 16 at 256 x 256 13.9, 15.3, at
-// 240 x 344 19.2, 16.7.  Wider boxes are the faster at every size.
-XBG_PLAN bool conv_rows_pays(int bn, int wc, long long pixels, int sms) {
-    return wc > 16 || pixels >= (bn == 16 ? 4LL : 3LL) * PLAN_GM * sms;
+// 16-channel boxes (32 bytes a pixel, so three times the boxes of a 48-channel input)
+// pay only where a CTA has rows enough; below, k_conv_tma's and k_conv_tc's blocks,
+// two and more to an SM, end first.  From three rows a CTA on for 16 -> 32 channels
+// (256 x 256 pixels 10.5 us there, 10.2 here; 512 x 1024 50.9, 32.8), from seven for
+// 16 -> 16 (256 x 512 12.3, 12.7; 4 x 192 x 192 17.9, 16.3), from six for 48 and 80
+// channels (48 -> 48 at 304 x 300 23.4, 27.1; at 256 x 512 32.2, 27.2), not at all
+// for these with 16 outputs (256 x 512 22.2, 26.5; 512 x 1024 74.4, 72.0), nor where
+// more than a fifth of their strips lies outside the image (48 -> 32 at 4 x 192 x 192
+// 31.6, 34.8).  Wider boxes are the faster at every size.
+XBG_PLAN bool conv_rows_pays(int bn, int cin, int W, long long pixels, int sms) {
+    if (cin % 32 == 0) return true;
+    if (cin > 16 && (bn == 16 || 4 * ((W + PLAN_GM - 1) / PLAN_GM) * PLAN_GM > 5 * W)) return false;
+    const long long rows = cin > 16 ? 6 : (bn == 16 ? 7 : 3);
+    return pixels >= rows * PLAN_GM * sms;
 }
 // A CTA's run: `per` consecutive output rows of the S = images x strips strips of H
 // rows, `cps` CTAs to a strip, or runs on end across strips (cps 0).  A run of n

@@ -1180,7 +1180,7 @@ int conv_launch(const void* X, const void* Wt, const float* bias, void* Y, int B
             if (cin % 32 == 0 && (nst = conv_rows_stages(BN, 32, W, cin)) &&
                 conv_map<32>(X, Bn, H, W, cin, ldx, &m, true))
                 return conv_rows_launch<BN, 32>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, dev, sms, err, st);
-            if (cin % 32 != 0 && cin % 16 == 0 && conv_rows_pays(BN, 16, M, sms) &&
+            if (cin % 32 != 0 && cin % 16 == 0 && conv_rows_pays(BN, cin, W, M, sms) &&
                 (nst = conv_rows_stages(BN, 16, W, cin)) &&
                 conv_map<16>(X, Bn, H, W, cin, ldx, &m, true))
                 return conv_rows_launch<BN, 16>(m, Wt, bias, Y, Bn, H, W, cin, ldw, ldy, flags, nst, dev, sms, err, st);
