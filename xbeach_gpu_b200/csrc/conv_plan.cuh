@@ -74,7 +74,7 @@ XBG_PLAN bool conv_rows_pays(int bn, int cin, int W, long long pixels, int sms) 
 // rows, `cps` CTAs to a strip, or runs on end across strips (cps 0).  A run of n
 // rows in one strip reads n + 2 input rows, one that crosses into the next strip
 // n + 4, so runs keep to a strip where that makes them no longer, or one row longer
-// in a layer whose time is its copies (extra).  48 -> 48 channels at 160 x 176 pixels
+// in a layer whose time is its copies (extra).  With waits by single lanes 48 -> 48 channels at 160 x 176 pixels
 // 19.9 us with runs across strips, 14.7 without; 32 -> 32 at 2 x 256 x 256 13.0, 11.1
 // (7 rows either way); 96 -> 32 at 240 x 1016 36.7, 34.4 (13 rows, 14); where products
 // bound the layer 14 rows for 13 lose: 64 -> 128 there 36.7, 38.2.

@@ -781,9 +781,9 @@ __device__ __forceinline__ void store_cols(unsigned taddr, const float* bias, vo
 // wait is bounded: a role that gives up sets a flag that ends the others' waits;
 // once every role has ended, the flag is final, and with it set the CTA leaves
 // after all its copies and products in flight (bounded again).
-// At 512 x 1024 pixels, against k_conv_tma: 32 -> 32 channels 64 -> 30 us, 96 -> 32
-// 146 -> 64, 16 -> 32 51 -> 25; at 256 x 512, 64 -> 64 38 -> 18.  What is left is
-// the issue of the products: 55 to 90 cycles each at 16 to 64 output channels.
+// At 512 x 1024 pixels, against k_conv_tma: 32 -> 32 channels 64 -> 36 us, 96 -> 32
+// 146 -> 85, 16 -> 32 51 -> 33; at 256 x 512, 64 -> 64 38 -> 19.  Waits by single
+// lanes took 30, 64, 25 and 18, but blocks bound by their stores faulted with them.
 constexpr int CR_THREADS = 192;
 
 template <int BN, int WC>
